@@ -664,7 +664,8 @@ int pg_upload(pg_ctx* c) {
   }
   for (int b = 0; b < 4; ++b) {
     PG_TRY(upload(c, s.rp[b], &P.rp[b]));
-    PG_TRY(dalloc(c, s.ci[b].size(), &P.val[b]));
+    // (two more than there are: the solver's copies of value ranges end on 16-byte boundaries)
+    PG_TRY(dalloc(c, s.ci[b].size() + 2, &P.val[b]));
   }
   // The values a later assembly can change (PG_KEEP_STATIC, pg_changing_values): every bulk law
   // is linear elastic, so only the entries coupling DOFs of nodes on one cohesive element depend
@@ -862,7 +863,7 @@ void pg_destroy(pg_ctx* c) {
   if (c->side2) cudaStreamSynchronize(c->side2);
   if (c->pcg.stream) cudaStreamSynchronize(c->pcg.stream);
   if (c->pcg.stream) cudaStreamDestroy(c->pcg.stream);
-  if (c->pcg.ev) cudaEventDestroy(c->pcg.ev);
+  for (cudaEvent_t e : {c->pcg.ev, c->pcg.evc[0], c->pcg.evc[1]}) if (e) cudaEventDestroy(e);
   if (c->pcg.hflag) cudaFreeHost(c->pcg.hflag);
   for (int i = 0; i < 6; ++i) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->side) cudaStreamDestroy(c->side);

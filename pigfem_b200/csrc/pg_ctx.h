@@ -16,17 +16,20 @@ namespace pgd { struct Tile3Const; }
 
 // Workspace of the Jacobi-preconditioned CG on K_ff (pg_solver.cu), allocated on first use.
 struct PcgWork {
-  int n = 0, cap_rhs = 0, nb = 0;
+  int cap_rhs = 0, nb = 0, ng = 0;              // right-hand sides of the buffers, blocks, row groups
+  int4* grp = nullptr;                          // row groups of K_ff (pg_solver.cu)
+  int* gci = nullptr;                           // their column lists
+  int4* chunk = nullptr;                        // chunks of groups: a warp's unit of work
+  int* part_of = nullptr;                       // nb + 1: the chunks of each block
   double* dinv = nullptr;                       // n: inverse diagonal of K_ff
-  const int* ci = nullptr;                      // column indices of K_ff
-  double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;  // cap_rhs x n each
+  double *r = nullptr, *p = nullptr, *q = nullptr, *xi = nullptr;   // n x cap_rhs each, interleaved
   double* part = nullptr;                       // partial sums: 3 x cap_rhs x nb
   double* sc = nullptr;                         // scalars per rhs (see pg_solver.cu)
-  int* flag = nullptr;                          // per rhs: done, iterations; [2*cap_rhs] = active count
-  int* hflag = nullptr;                         // pinned host copy of flag
+  int* flag = nullptr;                          // per rhs: done, iterations; then the solve's words
+  unsigned* bar = nullptr;                      // grid barrier arrivals
+  int* hflag = nullptr;                         // pinned host copies of flag (two launches in flight)
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev = nullptr;
-  bool diag_ready = false;
+  cudaEvent_t ev = nullptr, evc[2] = {nullptr, nullptr};
 };
 
 struct pg_ctx {

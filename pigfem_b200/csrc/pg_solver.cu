@@ -5,37 +5,750 @@
 //                  correction).  FP64 throughout; every inner product is a fixed-order reduction
 //                  (block partials over fixed row ranges, then one ordered sum), so a right-hand
 //                  side's iterates do not depend on the other right-hand sides solved with it, and
-//                  each right-hand side stops updating at its own convergence.  The iteration body
-//                  is captured once into a CUDA graph and replayed in chunks; the host reads one
-//                  flag word per chunk.
+//                  each right-hand side stops updating at its own convergence.  The iterations run
+//                  in cooperative launches of one block per SM, one launch ahead of the flags the
+//                  host has read.
 //   pg_homogenize  volume average of the stress over the volumetric quadrature points
 //                  (Problem::homogenize, src/Problem.cpp:471-484, with the stress functor of
 //                  include/AssemblerSmallStrainStructural.h:31-60).
 #include "pg_ctx.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kRowGroup = 8;          // lanes per CSR row in the matrix-vector product
-constexpr int kChunk = 16;            // iterations per graph replay
+constexpr int kThreads = 256;         // homogenization
+constexpr int kPcgThreads = 512;      // one block per SM: 128 registers a thread for 3 rows x 6 right-hand sides
+constexpr int kPcgWarps = kPcgThreads / 32;
+constexpr int kMaxRhs = 6;            // right-hand sides of one pass (the unit strains of a 3D homogenization)
+constexpr int kRound = 16;            // the host's iteration limit is a multiple of this
+constexpr unsigned kSpinLimit = 1u << 23;   // polls of one grid barrier (seconds) before it gives up
 // scalar slots per right-hand side in PcgWork::sc
-enum { S_RZ = 0, S_PQ, S_RR, S_BB, S_ALPHA, S_BETA, S_RELRES, S_NSC };
+enum { S_RZ = 0, S_BB, S_RELRES, S_NSC };
+// word slots after the 2 x NS per-right-hand-side words of PcgWork::flag
+enum { F_ACTIVE = 0, F_BAD, F_STUCK, F_N };
+
+// The matrix reaches the product through shared memory: a warp's unit of work is a chunk of up to
+// 32 / L consecutive row groups whose values, columns and descriptors fit one stage, fetched by
+// bulk copies into the warp's own ring of stages.  A chunk too long for a stage (kDirect) is read
+// from global memory.
+template <int M> struct PcgShape;
+template <> struct PcgShape<2> {   // 2D: 8 groups of two rows, about 2.3 KB
+  static constexpr int L = 4, kGroups = 8, kColBytes = 608, kValBytes = 2464, kStages = 4;
+};
+template <> struct PcgShape<3> {   // 3D: 4 groups of three rows of 45, 5.1 KB
+  static constexpr int L = 8, kGroups = 4, kColBytes = 912, kValBytes = 5424, kStages = 2;
+};
+template <int M>
+__host__ __device__ constexpr int pcg_stage_bytes() {
+  return PcgShape<M>::kGroups * 16 + PcgShape<M>::kColBytes + PcgShape<M>::kValBytes;
+}
+template <int M>
+constexpr int pcg_smem_bytes() { return kPcgWarps * PcgShape<M>::kStages * (pcg_stage_bytes<M>() + 8); }
+static_assert(pcg_stage_bytes<2>() % 16 == 0 && pcg_stage_bytes<3>() % 16 == 0, "bulk copies need 16-byte stages");
+static_assert(PcgShape<2>::kColBytes % 16 == 0 && PcgShape<3>::kColBytes % 16 == 0, "16-byte parts");
+
+// word w of a group: row length, rows << 24, kDirect, groups of its chunk from this one on << 28
+constexpr unsigned kDirect = 1u << 26;
+__host__ __device__ constexpr int grp_len(unsigned w) { return (int)(w & 0xffffffu); }
+__host__ __device__ constexpr int grp_rows(unsigned w) { return (int)(w >> 24) & 3; }
 
 struct PcgArgs {
-  const int* rp;
-  const int* ci;
+  const int4* grp;        // row groups: {first row, first value, first entry of gci, w}
+  const int* gci;         // one column list per group (its rows share it)
+  const int4* chunk;      // chunks: {first group, groups, first value, first entry of gci}, and the end
+  const int* part_of;     // nb + 1: the chunks of each block
   const double* val;
-  int n, nrhs, nb;
+  int n, ng, nb;
   double rtol;
-  const double* dinv;
-  double *x, *r, *z, *p, *q;   // p interleaved by right-hand side: p[i * nrhs + s]; the others [s][n]
-  double* part;   // [3][nrhs][nb]
-  double* sc;     // [nrhs][S_NSC]
-  int* flag;      // [0, nrhs) done, [nrhs, 2 nrhs) iterations, [2 nrhs] active count
+  const double* b;        // [s][n]
+  double* x;              // [s][n]
+  double *dinv, *r, *p, *q, *xi;   // r, p, q, xi (the iterates) interleaved by right-hand side: [i * NS + s]
+  double* part;           // [2 NS + NS][nb] partial sums
+  double* sc;             // [NS][S_NSC]
+  int* flag;              // [0, NS) done, [NS, 2 NS) iterations, then F_*
+  unsigned* bar;          // arrivals at the grid barriers of this solve
 };
+
+// NS adjacent doubles (16-byte pairs when NS is even).  Plain loads: p and q change during the
+// kernel, and the grid barrier's acquire makes the other blocks' values visible.
+template <int NS>
+__device__ __forceinline__ void load_ns(const double* p, size_t i, double* out) {
+  if constexpr (NS % 2 == 0) {
+    const double2* q = reinterpret_cast<const double2*>(p + i * NS);
+#pragma unroll
+    for (int j = 0; j < NS / 2; ++j) { const double2 t = q[j]; out[2 * j] = t.x; out[2 * j + 1] = t.y; }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NS; ++j) out[j] = p[i * NS + j];
+  }
+}
+template <int NS>
+__device__ __forceinline__ void store_ns(double* p, size_t i, const double* v) {
+  if constexpr (NS % 2 == 0) {
+    double2* q = reinterpret_cast<double2*>(p + i * NS);
+#pragma unroll
+    for (int j = 0; j < NS / 2; ++j) q[j] = make_double2(v[2 * j], v[2 * j + 1]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < NS; ++j) p[i * NS + j] = v[j];
+  }
+}
+
+// Before the first pass of a solve: the inverse diagonal (the matrix changes with every assembly)
+// and the initial guess interleaved into p and xi.  A thread per row group.
+template <int NS>
+__global__ void __launch_bounds__(128) k_pcg_prepare(PcgArgs a) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= a.ng) return;
+  const int4 d = __ldg(&a.grp[g]);
+  const int len = grp_len(d.w), m = grp_rows(d.w);
+  for (int i = 0; i < m; ++i) {
+    const int row = d.x + i;
+    // the columns are sorted: the group's rows are its own columns, so the diagonal is found by bisection
+    int lo = 0, hi = len;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(&a.gci[d.z + mid]) < row) lo = mid + 1; else hi = mid;
+    }
+    const double v = (lo < len && __ldg(&a.gci[d.z + lo]) == row) ? __ldg(&a.val[d.y + i * len + lo]) : 0.0;
+    if (!(v > 0.0) || !isfinite(v)) { atomicOr(&a.flag[2 * NS + F_BAD], 1); a.dinv[row] = 0.0; }
+    else a.dinv[row] = 1.0 / v;
+    double xv[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) xv[s] = a.x[(size_t)s * a.n + row];
+    store_ns<NS>(a.p, row, xv);
+    store_ns<NS>(a.xi, row, xv);
+  }
+}
+
+// After the last iteration: the solutions into the caller's layout.
+template <int NS>
+__global__ void __launch_bounds__(128) k_pcg_finish(PcgArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  double xv[NS];
+  load_ns<NS>(a.xi, i, xv);
+#pragma unroll
+  for (int s = 0; s < NS; ++s) a.x[(size_t)s * a.n + i] = xv[s];
+}
+
+// Sums of C values over the lanes of a warp, scattered: at each step a lane hands half of its
+// values to its partner and keeps the other half, so C values cost about C shuffles instead of
+// 5 C.  Every value's additions form the butterfly tree l ^ 16, l ^ 8, ..., whichever lane ends up
+// with it, so a value's sum does not depend on C.  Returns the index of the value left in v[0].
+template <int C, int O>
+__device__ __forceinline__ int scatter_sum(double* v, int lane) {
+  if constexpr (O == 0) {
+    return 0;
+  } else {
+    constexpr int H = (C + 1) / 2;
+    const bool up = (lane & O) != 0;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const double lo = v[i], hi = (i + H < C) ? v[i + H] : v[i];
+      const double got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, O);
+      v[i] = __dadd_rn(up ? hi : lo, got);
+    }
+    const int k = scatter_sum<H, O / 2>(v, lane);
+    return (up && k + H < C) ? k + H : k;
+  }
+}
+
+// The block's sums of C per-thread values to part[k * nb + block], in a fixed order.
+template <int C>
+__device__ __forceinline__ void block_sums(double* v, double (*red)[3 * kMaxRhs], double* part, int nb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = scatter_sum<C, 16>(v, lane);
+  red[warp][k] = v[0];   // lanes left with the same value hold the same bits
+  __syncthreads();
+  if (threadIdx.x < C) {
+    double t = red[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < kPcgWarps; ++w) t = __dadd_rn(t, red[w][threadIdx.x]);
+    part[threadIdx.x * nb + blockIdx.x] = t;
+  }
+}
+
+// All blocks of the (cooperative) launch meet: the arrivals of a solve are counted in one word
+// that only grows, `target` is its value once every block has arrived.  Bounded: false once the
+// limit is reached (the caller returns and the host reports it).
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* stuck) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    unsigned got, spins = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(bar) : "memory");
+    } while ((int)(got - target) < 0 && ++spins < kSpinLimit);
+    ok = (int)(got - target) >= 0;
+    if (!ok) atomicOr(stuck, 1);
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Ordered sums of the blocks' partials of C values: tot[k], the same in every block.
+template <int C>
+__device__ __forceinline__ void total_sums(const double* part, int nb, double* tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = warp; k < C; k += kPcgWarps) {
+    double t = 0.0;
+    for (int i = lane; i < nb; i += 32) t = __dadd_rn(t, part[k * nb + i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+    if (lane == 0) tot[k] = t;
+  }
+  __syncthreads();
+}
+
+// A warp's ring of stages.  The chunks of the warp follow each other through the iterations (the
+// matrix does not change), so the first chunks of the next product are fetched while the vectors
+// are updated; when all of them fit the ring they are fetched once.
+template <int M>
+struct PcgRing {
+  using S = PcgShape<M>;
+  unsigned char* mem;       // the warp's stages
+  unsigned bar;             // shared address of the warp's barriers
+  const int4* first;        // the warp's first chunk; the following are kPcgWarps apart
+  int n;                    // its chunks
+  bool resident;
+  unsigned issued, used;    // chunks fetched / consumed so far
+
+  __device__ __forceinline__ void issue(const PcgArgs& a) {   // one lane
+    const int4 c = __ldg(first + (size_t)(issued % n) * kPcgWarps), e = __ldg(first + (size_t)(issued % n) * kPcgWarps + 1);
+    const unsigned st = issued % S::kStages;
+    const unsigned full = bar + 8 * st;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(mem + st * pcg_stage_bytes<M>());
+    const bool direct = (c.y & 256) != 0;
+    const int v0 = c.z & ~1, c0 = c.w & ~3;
+    const unsigned gb = (c.y & 255) * 16u;
+    const unsigned vb = direct ? 0u : (unsigned)(((e.z + 1) & ~1) - v0) * 8u;
+    const unsigned cb = direct ? 0u : (unsigned)(((e.w + 3) & ~3) - c0) * 4u;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(gb + vb + cb) : "memory");
+    auto copy = [&](unsigned to, const void* from, unsigned bytes) {
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
+                   "l"(from), "r"(bytes), "r"(full)
+                   : "memory");
+    };
+    copy(dst, a.grp + c.x, gb);
+    if (cb) copy(dst + S::kGroups * 16, a.gci + c0, cb);
+    if (vb) copy(dst + S::kGroups * 16 + S::kColBytes, a.val + v0, vb);
+  }
+  // Waits (bounded) for stage st's fetch number `turn`; the whole warp calls it and agrees.
+  __device__ __forceinline__ bool wait(unsigned st, unsigned turn) const {
+    for (unsigned k = 0; k < kSpinLimit; ++k) {
+      unsigned ok;
+      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                   : "=r"(ok) : "r"(bar + 8 * st), "r"(turn & 1u) : "memory");
+      if (__all_sync(0xffffffffu, ok)) return true;
+    }
+    return false;
+  }
+  __device__ __forceinline__ void fill(const PcgArgs& a, int lane) {
+    const unsigned upto = resident ? (unsigned)n : used + S::kStages;
+    for (; n > 0 && issued < upto; ++issued)
+      if (lane == 0) issue(a);
+  }
+  // Waits for every fetch still in flight (before the block returns).
+  __device__ __forceinline__ void drain() {
+    if (resident) { for (unsigned k = 0; used == 0 && k < issued; ++k) wait(k, 0); return; }
+    for (; used < issued; ++used) wait(used % S::kStages, used / S::kStages);
+  }
+};
+
+// q = A p on the block's rows, L lanes per row group (a node's free DOFs: up to M consecutive rows
+// with one column list).  A lane takes the nonzeros lane, lane + L, ... of all the group's rows, so
+// a column index and a column's NS values of p are read once for M rows; the lanes' sums are then
+// exchanged so that each row ends in its own lane.  A row's products and sums are the same for any
+// NS.  pq gets the lane's rows' p.q.  false when a fetch did not arrive.
+template <int NS, int M>
+__device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring, double* pq) {
+  using S = PcgShape<M>;
+  constexpr int L = S::L;
+  const int wl = threadIdx.x & 31, lane = wl % L, sub = wl / L;
+#pragma unroll
+  for (int j = 0; j < NS; ++j) pq[j] = 0.0;
+  for (int i = 0; i < ring.n; ++i) {
+    const unsigned st = ring.resident ? (unsigned)i : ring.used % S::kStages;
+    if (!ring.wait(st, ring.resident ? 0u : ring.used / S::kStages)) return false;
+    const unsigned char* mem = ring.mem + st * pcg_stage_bytes<M>();
+    const int4* sg = reinterpret_cast<const int4*>(mem);
+    const int4 d0 = sg[0];
+    int4 d = make_int4(0, 0, 0, 0);
+    if (sub < (int)((unsigned)d0.w >> 28)) d = sg[sub];
+    const int len = grp_len(d.w), m = grp_rows(d.w);
+    // the row this lane ends up with, and its own p
+    int mine;
+    if constexpr (M == 3) mine = (lane & 4) ? 2 : ((lane & 2) ? 1 : 0);
+    else mine = (lane & 2) ? 1 : 0;
+    const bool writer = (M == 3 ? (lane == 0 || lane == 2 || lane == 4) : (lane == 0 || lane == 2)) && mine < m;
+    double own[NS];
+    if (writer) load_ns<NS>(a.p, d.x + mine, own);
+    double acc[M][NS];
+#pragma unroll
+    for (int r = 0; r < M; ++r)
+#pragma unroll
+      for (int j = 0; j < NS; ++j) acc[r][j] = 0.0;
+    auto rows = [&](const double* v, const int* ci) {
+#pragma unroll 3
+      for (int k = lane; k < len; k += L) {
+        double av[M], pv[NS];
+        load_ns<NS>(a.p, ci[k], pv);
+#pragma unroll
+        for (int r = 0; r < M; ++r) av[r] = (r < m) ? v[r * len + k] : 0.0;
+#pragma unroll
+        for (int r = 0; r < M; ++r)
+#pragma unroll
+          for (int j = 0; j < NS; ++j) acc[r][j] = __fma_rn(av[r], pv[j], acc[r][j]);
+      }
+    };
+    if ((unsigned)d0.w & kDirect) {
+      rows(a.val + d.y, a.gci + d.z);
+    } else {
+      const int* sc = reinterpret_cast<const int*>(mem + S::kGroups * 16);
+      const double* sv = reinterpret_cast<const double*>(mem + S::kGroups * 16 + S::kColBytes);
+      rows(sv + (d.y - (d0.y & ~1)), sc + (d.z - (d0.z & ~3)));
+    }
+    __syncwarp();   // the stage is read
+    if (!ring.resident) {
+      ++ring.used;
+      ring.fill(a, wl);
+    }
+    double qv[NS];
+    if constexpr (M == 3) {
+      const bool hi = (lane & 4) != 0, odd = (lane & 2) != 0;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const double got0 = __shfl_xor_sync(0xffffffffu, hi ? acc[0][j] : acc[2][j], 4);
+        const double x = __dadd_rn(hi ? acc[2][j] : acc[0][j], got0);
+        const double y = __dadd_rn(acc[1][j], __shfl_xor_sync(0xffffffffu, acc[1][j], 4));
+        const double got = __shfl_xor_sync(0xffffffffu, (hi || odd) ? x : y, 2);
+        const double t = __dadd_rn((!hi && odd) ? y : x, got);
+        qv[j] = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 1));
+      }
+    } else {
+      const bool hi = (lane & 2) != 0;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const double got = __shfl_xor_sync(0xffffffffu, hi ? acc[0][j] : acc[1][j], 2);
+        const double t = __dadd_rn(hi ? acc[1][j] : acc[0][j], got);
+        qv[j] = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 1));
+      }
+    }
+    if (writer) {
+      store_ns<NS>(a.q, d.x + mine, qv);
+#pragma unroll
+      for (int j = 0; j < NS; ++j) pq[j] = __fma_rn(own[j], qv[j], pq[j]);
+    }
+  }
+  if (ring.resident) ring.used = 1;   // fetched and seen
+  return true;
+}
+
+// Iterations [it0, it1) of the solve in one cooperative launch, one block per SM, each block owning
+// a fixed range of rows with about the same number of nonzeros.  Per iteration three passes over
+// the block's rows, separated by grid barriers:
+//   q = A p, partial p.q  |  r -= alpha q, partials of r.z and r.r (z = D^-1 r is never stored)
+//   |  x += alpha p, p = z + beta p  |
+// Every block forms the scalars itself from all blocks' partials, in the same order, so the blocks
+// agree on them and on who is done.  `first`: r = b - A x, p = z before the iterations.
+// One launch per round instead of five kernels per iteration: a 128 x 128 tri3 RVE with three
+// right-hand sides (39,614 rows) takes 11.4 us per iteration (five kernels: 36 us), of which the
+// three barriers with their scalars are about 5 us; 40^3 tet4 with six (219,807 rows, 9.7 M
+// nonzeros) 65 us (134 us), bound by the latency and L1 wavefronts of the gathers of p (48 bytes
+// per lane) at 16 warps per SM.
+template <int NS, int M>
+__global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first, int it0, int it1, unsigned arrived) {
+  __shared__ double red[kPcgWarps][3 * kMaxRhs];
+  __shared__ double tot[3 * kMaxRhs];
+  __shared__ double rz[kMaxRhs], bb[kMaxRhs], relres[kMaxRhs], step[kMaxRhs], coef[kMaxRhs];
+  __shared__ int done[kMaxRhs], iters[kMaxRhs], active;
+  const int t = threadIdx.x;
+  if (a.flag[2 * NS + F_BAD]) return;   // set before this launch
+  extern __shared__ __align__(16) unsigned char stages[];
+  const int c0 = __ldg(&a.part_of[blockIdx.x]), c1 = __ldg(&a.part_of[blockIdx.x + 1]);
+  int r0 = 0, r1 = 0;
+  if (c0 < c1) {
+    r0 = __ldg(&a.grp[__ldg(&a.chunk[c0]).x]).x;
+    const int4 d = __ldg(&a.grp[__ldg(&a.chunk[c1]).x - 1]);
+    r1 = d.x + grp_rows(d.w);
+  }
+  PcgRing<M> ring;
+  {
+    using S = PcgShape<M>;
+    const int warp = t >> 5;
+    ring.mem = stages + (size_t)warp * S::kStages * pcg_stage_bytes<M>();
+    unsigned char* bars = stages + (size_t)kPcgWarps * S::kStages * pcg_stage_bytes<M>();
+    ring.bar = (unsigned)__cvta_generic_to_shared(bars) + 8u * S::kStages * warp;
+    ring.first = a.chunk + c0 + warp;
+    ring.n = (c1 - c0 - warp + kPcgWarps - 1) / kPcgWarps;
+    if (ring.n < 0) ring.n = 0;
+    ring.resident = ring.n <= S::kStages;
+    ring.issued = ring.used = 0;
+    if ((t & 31) == 0) {
+      for (int k = 0; k < S::kStages; ++k)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring.bar + 8u * k) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    ring.fill(a, t & 31);
+  }
+  unsigned target = arrived;
+  int* stuck = &a.flag[2 * NS + F_STUCK];
+  bool fine = true;
+  double sum[2 * NS + NS];
+  // a barrier or a fetch that gave up: the block waits for its own copies and returns
+  auto give_up = [&]() {
+    if (!fine) atomicOr(stuck, 1);
+    ring.drain();
+  };
+  if (first) {
+    fine = block_product<NS, M>(a, ring, sum);
+    if (!__syncthreads_and(fine)) { give_up(); return; }   // (and the block's q)
+#pragma unroll
+    for (int k = 0; k < 3 * NS; ++k) sum[k] = 0.0;
+    for (int i = r0 + t; i < r1; i += kPcgThreads) {
+      double qv[NS], rv[NS];
+      load_ns<NS>(a.q, i, qv);
+      const double di = a.dinv[i];
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const double bj = a.b[(size_t)j * a.n + i];
+        rv[j] = __dsub_rn(bj, qv[j]);
+        sum[j] = __fma_rn(rv[j], __dmul_rn(di, rv[j]), sum[j]);
+        sum[NS + j] = __fma_rn(rv[j], rv[j], sum[NS + j]);
+        sum[2 * NS + j] = __fma_rn(bj, bj, sum[2 * NS + j]);
+      }
+      store_ns<NS>(a.r, i, rv);
+    }
+    block_sums<3 * NS>(sum, red, a.part, a.nb);
+    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    total_sums<3 * NS>(a.part, a.nb, tot);
+    if (t == 0) {
+      active = 0;
+      for (int j = 0; j < NS; ++j) {
+        const double nb2 = sqrt(tot[2 * NS + j]);
+        rz[j] = tot[j];
+        bb[j] = tot[2 * NS + j];
+        relres[j] = nb2 > 0.0 ? sqrt(tot[NS + j]) / nb2 : 0.0;
+        done[j] = (nb2 == 0.0) || (relres[j] <= a.rtol);
+        iters[j] = 0;
+        active += !done[j];
+      }
+    }
+    for (int i = r0 + t; i < r1; i += kPcgThreads) {
+      double rv[NS];
+      load_ns<NS>(a.r, i, rv);
+      const double di = a.dinv[i];
+#pragma unroll
+      for (int j = 0; j < NS; ++j) rv[j] = __dmul_rn(di, rv[j]);
+      store_ns<NS>(a.p, i, rv);
+    }
+    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+  } else {
+    if (t < NS) {
+      rz[t] = a.sc[t * S_NSC + S_RZ];
+      bb[t] = a.sc[t * S_NSC + S_BB];
+      relres[t] = a.sc[t * S_NSC + S_RELRES];
+      done[t] = a.flag[t];
+      iters[t] = a.flag[NS + t];
+    }
+    if (t == 0) active = a.flag[2 * NS + F_ACTIVE];
+    __syncthreads();
+  }
+  for (int it = it0; it < it1 && active > 0; ++it) {
+    fine = block_product<NS, M>(a, ring, sum);
+    if (!__syncthreads_and(fine)) { give_up(); return; }
+    block_sums<NS>(sum, red, a.part, a.nb);
+    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    total_sums<NS>(a.part, a.nb, tot);
+    if (t < NS) step[t] = rz[t] / tot[t];
+    __syncthreads();
+    double al[NS];
+    bool act[NS];
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+      act[j] = !done[j];
+      al[j] = act[j] ? step[j] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * NS; ++k) sum[k] = 0.0;
+#pragma unroll 2
+    for (int i = r0 + t; i < r1; i += kPcgThreads) {
+      double qv[NS], rv[NS];
+      load_ns<NS>(a.q, i, qv);
+      load_ns<NS>(a.r, i, rv);
+      const double di = a.dinv[i];
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        if (act[j]) rv[j] = __fma_rn(-al[j], qv[j], rv[j]);
+        sum[j] = __fma_rn(rv[j], __dmul_rn(di, rv[j]), sum[j]);
+        sum[NS + j] = __fma_rn(rv[j], rv[j], sum[NS + j]);
+      }
+      store_ns<NS>(a.r, i, rv);
+    }
+    // (the second set of partials: a block may still be reading the first)
+    block_sums<2 * NS>(sum, red, a.part + NS * a.nb, a.nb);
+    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    total_sums<2 * NS>(a.part + NS * a.nb, a.nb, tot);
+    if (t < NS) {
+      coef[t] = tot[t] / rz[t];
+      if (!done[t]) {
+        rz[t] = tot[t];
+        relres[t] = sqrt(tot[NS + t]) / sqrt(bb[t]);
+        ++iters[t];
+      }
+    }
+    __syncthreads();
+    // x and p, element by element: the vectors are interleaved, so consecutive threads take
+    // consecutive words whatever NS is
+    constexpr int W = (NS % 2 == 0) ? 2 : 1;
+    double* const vx = a.xi + (size_t)r0 * NS;
+    double* const vp = a.p + (size_t)r0 * NS;
+    const double* const vr = a.r + (size_t)r0 * NS;
+    const int nw = (r1 - r0) * (NS / W);
+#pragma unroll 4
+    for (int e = t; e < nw; e += kPcgThreads) {
+      const int row = e / (NS / W), j0 = (e - row * (NS / W)) * W;
+      double xv[W], pv[W], rv[W];
+      load_ns<W>(vx, e, xv);
+      load_ns<W>(vp, e, pv);
+      load_ns<W>(vr, e, rv);
+      const double di = a.dinv[r0 + row];
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        if (!done[j0 + j]) {
+          xv[j] = __fma_rn(step[j0 + j], pv[j], xv[j]);
+          pv[j] = __fma_rn(coef[j0 + j], pv[j], __dmul_rn(di, rv[j]));
+        }
+      store_ns<W>(vx, e, xv);
+      store_ns<W>(vp, e, pv);
+    }
+    __syncthreads();   // everyone is past reading done
+    if (t == 0) {
+      int n_act = 0;
+      for (int j = 0; j < NS; ++j) {
+        if (!done[j] && (relres[j] <= a.rtol || !isfinite(relres[j]))) done[j] = 1;
+        n_act += !done[j];
+      }
+      active = n_act;
+    }
+    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+  }
+  ring.drain();
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    if (t < NS) {
+      a.sc[t * S_NSC + S_RZ] = rz[t];
+      a.sc[t * S_NSC + S_BB] = bb[t];
+      a.sc[t * S_NSC + S_RELRES] = relres[t];
+      a.flag[t] = done[t];
+      a.flag[NS + t] = iters[t];
+    }
+    if (t == 0) a.flag[2 * NS + F_ACTIVE] = active;
+  }
+}
+
+struct PcgKernels {
+  void (*run)(PcgArgs, int, int, int, unsigned);
+  void (*prepare)(PcgArgs);
+  void (*finish)(PcgArgs);
+  int smem;
+};
+template <int NS>
+PcgKernels pcg_kernels(int dim) {
+  if (dim == 3) return {k_pcg_run<NS, 3>, k_pcg_prepare<NS>, k_pcg_finish<NS>, pcg_smem_bytes<3>()};
+  return {k_pcg_run<NS, 2>, k_pcg_prepare<NS>, k_pcg_finish<NS>, pcg_smem_bytes<2>()};
+}
+
+// Row groups and chunks of K_ff: the consecutive rows of one DOF node share one column list.
+template <int M>
+void pcg_groups(const pg::Setup& s, std::vector<int4>& grp, std::vector<int>& gci, std::vector<int4>& chunk) {
+  using S = PcgShape<M>;
+  const int n = s.n_free;
+  const std::vector<int>& rp = s.rp[0];
+  std::vector<int> owner(n, -1);
+  for (int a = 0; a < s.n_dn; ++a)
+    for (int q = 0; q < s.dim; ++q) {
+      const int g = s.node_dof[(size_t)s.dn_node[a] * s.dim + q];
+      if (g < n) owner[g] = a;
+    }
+  grp.reserve(n / M + 1);
+  gci.reserve(s.ci[0].size() / M + 64);
+  int open = 0;   // groups of the open chunk
+  auto close = [&](bool direct) {
+    if (!open) return;
+    chunk.back().y = open | (direct ? 256 : 0);
+    for (int k = 0; k < open; ++k) {
+      int4& d = grp[grp.size() - open + k];
+      d.w = (int)((unsigned)d.w | (direct ? kDirect : 0u) | ((unsigned)(open - k) << 28));
+    }
+    open = 0;
+  };
+  for (int r = 0; r < n;) {
+    const int len = rp[r + 1] - rp[r];
+    int m = 1;
+    while (m < M && r + m < n && owner[r + m] == owner[r] && owner[r] >= 0 && rp[r + m + 1] - rp[r + m] == len) ++m;
+    const int v1 = rp[r + m], c1 = (int)gci.size() + len;
+    // (with the 16-byte boundaries the copies start and end on)
+    auto fits = [&](int v0, int c0) {
+      return (((v1 + 1) & ~1) - (v0 & ~1)) * 8 <= S::kValBytes && (((c1 + 3) & ~3) - (c0 & ~3)) * 4 <= S::kColBytes;
+    };
+    if (open == S::kGroups || (open && !fits(chunk.back().z, chunk.back().w))) close(false);
+    if (!open) chunk.push_back(make_int4((int)grp.size(), 0, rp[r], (int)gci.size()));
+    grp.push_back(make_int4(r, rp[r], (int)gci.size(), len | (m << 24)));
+    gci.insert(gci.end(), s.ci[0].begin() + rp[r], s.ci[0].begin() + rp[r + 1]);
+    ++open;
+    if (open == 1 && !fits(chunk.back().z, chunk.back().w)) close(true);   // longer than a stage: alone, read from global memory
+    r += m;
+  }
+  close(false);
+  chunk.push_back(make_int4((int)grp.size(), 0, n ? rp[n] : 0, (int)gci.size()));
+}
+
+int pcg_reserve(pg_ctx* c, int nrhs) {
+  PcgWork& w = c->pcg;
+  const pg::Setup& s = c->s;
+  const int n = s.n_free, dim = s.dim;
+  if (!w.stream) {
+    if (cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&w.ev, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&w.evc[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&w.evc[1], cudaEventDisableTiming) != cudaSuccess)
+      return pg_set_err(c, PG_ERR_DEVICE, "solver stream creation failed");
+    if (cudaMallocHost(&w.hflag, sizeof(int) * 64) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "pinned flag allocation failed");
+  }
+  int rc = 0;
+  if (!w.grp) {
+    std::vector<int4> grp, chunk;
+    std::vector<int> gci;
+    if (dim == 3) pcg_groups<3>(s, grp, gci, chunk);
+    else pcg_groups<2>(s, grp, gci, chunk);
+    for (const int4& d : grp)
+      if (grp_len(d.w) >= 0x1000000 - 1) return pg_set_err(c, PG_ERR_UNSUPPORTED, "a row of K_ff with 2^24 entries");
+    const int ng = (int)grp.size(), nch = (int)chunk.size() - 1;
+    // blocks: one per SM (the launch is cooperative), fewer when there are fewer chunks than
+    // warps; contiguous chunk ranges of about equal nonzeros plus vector work
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    w.nb = std::max(1, std::min(sms, (nch + kPcgWarps - 1) / kPcgWarps));
+    auto weight = [&](int k) { return (double)(chunk[k + 1].z - chunk[k].z) + 16.0 * dim * (chunk[k + 1].x - chunk[k].x); };
+    double total = 0.0, acc = 0.0;
+    for (int k = 0; k < nch; ++k) total += weight(k);
+    std::vector<int> part(w.nb + 1, nch);
+    part[0] = 0;
+    for (int k = 0, b = 1; k < nch && b < w.nb; ++k) {
+      acc += weight(k);
+      while (b < w.nb && acc >= total * b / w.nb) part[b++] = k + 1;
+    }
+    w.ng = ng;
+    gci.resize((gci.size() + 7) & ~(size_t)3);   // the last chunk's copy ends on a 16-byte boundary
+    rc |= pg_dalloc(c, grp.size(), &w.grp) | pg_dalloc(c, gci.size(), &w.gci) | pg_dalloc(c, chunk.size(), &w.chunk) |
+          pg_dalloc(c, part.size(), &w.part_of) | pg_dalloc(c, (size_t)n, &w.dinv) | pg_dalloc(c, 1, &w.bar);
+    if (rc) return PG_ERR_DEVICE;
+    if (cudaMemcpyAsync(w.grp, grp.data(), grp.size() * sizeof(int4), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
+        cudaMemcpyAsync(w.gci, gci.data(), gci.size() * sizeof(int), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
+        cudaMemcpyAsync(w.chunk, chunk.data(), chunk.size() * sizeof(int4), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
+        cudaMemcpyAsync(w.part_of, part.data(), part.size() * sizeof(int), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
+        pg_alloc_sync(c))
+      return pg_set_err(c, PG_ERR_DEVICE, "solver tables: copy failed");
+  }
+  if (w.cap_rhs < nrhs) {
+    // (a solve returns with its work done, so the smaller buffers are idle)
+    for (double* p : {w.r, w.p, w.q, w.xi, w.part, w.sc}) if (p) pg_untrack_free(c, p);
+    if (w.flag) pg_untrack_free(c, w.flag);
+    w.r = w.p = w.q = w.xi = w.part = w.sc = nullptr;
+    w.flag = nullptr;
+    w.cap_rhs = 0;
+    rc |= pg_dalloc(c, (size_t)n * nrhs, &w.r) | pg_dalloc(c, (size_t)n * nrhs, &w.p) | pg_dalloc(c, (size_t)n * nrhs, &w.q) |
+          pg_dalloc(c, (size_t)n * nrhs, &w.xi) | pg_dalloc(c, (size_t)3 * nrhs * w.nb, &w.part) | pg_dalloc(c, (size_t)S_NSC * nrhs, &w.sc) |
+          pg_dalloc(c, (size_t)2 * nrhs + F_N, &w.flag);
+    if (rc) return PG_ERR_DEVICE;
+    w.cap_rhs = nrhs;
+    return pg_alloc_sync(c);
+  }
+  return 0;
+}
+
+// Solves for NS = nrhs <= kMaxRhs right-hand sides; *all is cleared when one misses the tolerance.
+int pcg_pass(pg_ctx* c, const double* d_b, double* d_x, int nrhs, double rtol, int max_it, int* iters, double* relres,
+             bool* all) {
+  PcgWork& w = c->pcg;
+  const int n = c->s.n_free;
+  PcgArgs a{w.grp, w.gci, w.chunk, w.part_of, c->P.val[0], n, w.ng, w.nb, rtol, d_b, d_x,
+            w.dinv, w.r, w.p, w.q, w.xi, w.part, w.sc, w.flag, w.bar};
+  PcgKernels k;
+  switch (nrhs) {
+    case 1: k = pcg_kernels<1>(c->s.dim); break;
+    case 2: k = pcg_kernels<2>(c->s.dim); break;
+    case 3: k = pcg_kernels<3>(c->s.dim); break;
+    case 4: k = pcg_kernels<4>(c->s.dim); break;
+    case 5: k = pcg_kernels<5>(c->s.dim); break;
+    default: k = pcg_kernels<6>(c->s.dim); break;
+  }
+  if (cudaFuncSetAttribute((const void*)k.run, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem) != cudaSuccess)
+    return pg_set_err(c, PG_ERR_DEVICE, "solver shared memory request failed");
+  const int n_flag = 2 * nrhs + F_N;
+  cudaMemsetAsync(w.flag, 0, sizeof(int) * n_flag, w.stream);
+  cudaMemsetAsync(w.bar, 0, sizeof(unsigned), w.stream);
+  k.prepare<<<(w.ng + 127) / 128, 128, 0, w.stream>>>(a);
+  // Launches of `chunk` iterations, one ahead of the flags the host has seen (a launch that finds
+  // every right-hand side done returns at once).  Short iterations get longer launches, so the
+  // launch and its scalars' reload stay small beside them; long ones keep the default round, so
+  // other streams' work gets its turn within a millisecond or two.
+  const int limit = (int)std::min<long long>(((long long)max_it + kRound - 1) / kRound * kRound, 2147483647LL / kRound * kRound);
+  const int chunk = ((double)c->s.ci[0].size() * (2 + nrhs) < 2e7) ? 8 * kRound : kRound;
+  unsigned arrived = 0;
+  int it = 0, rc = 0;
+  for (int l = 0;; ++l) {
+    if (it < limit) {
+      int first = l == 0, it0 = it, it1 = std::min(limit, it + chunk);
+      void* args[] = {&a, &first, &it0, &it1, &arrived};
+      if (cudaLaunchCooperativeKernel((const void*)k.run, dim3(w.nb), dim3(kPcgThreads), args, (size_t)k.smem, w.stream) != cudaSuccess) {
+        rc = pg_set_err(c, PG_ERR_DEVICE, "solver launch failed");
+        break;
+      }
+      arrived += (unsigned)(w.nb * (3 * (it1 - it0) + (first ? 2 : 0)));
+      it = it1;
+    }
+    cudaMemcpyAsync(w.hflag + 32 * (l & 1), w.flag, sizeof(int) * n_flag, cudaMemcpyDeviceToHost, w.stream);
+    cudaEventRecord(w.evc[l & 1], w.stream);
+    if (l == 0 && it < limit) continue;
+    // the flags of the launch before this one (of this one when it is the last)
+    const int look = it < limit ? (l - 1) & 1 : l & 1;
+    if (cudaEventSynchronize(w.evc[look]) != cudaSuccess) { rc = pg_set_err(c, PG_ERR_DEVICE, "solver iteration failed"); break; }
+    const int* f = w.hflag + 32 * look + 2 * nrhs;
+    if (f[F_BAD] || f[F_STUCK] || f[F_ACTIVE] == 0 || it >= limit) break;
+  }
+  std::vector<double> sc((size_t)S_NSC * nrhs);
+  if (!rc) {
+    // (a bad diagonal leaves the caller's x as it was: xi still holds it)
+    k.finish<<<(n + 127) / 128, 128, 0, w.stream>>>(a);
+    cudaMemcpyAsync(sc.data(), w.sc, sizeof(double) * sc.size(), cudaMemcpyDeviceToHost, w.stream);
+    cudaMemcpyAsync(w.hflag, w.flag, sizeof(int) * n_flag, cudaMemcpyDeviceToHost, w.stream);
+  }
+  if (cudaStreamSynchronize(w.stream) != cudaSuccess && !rc) rc = pg_set_err(c, PG_ERR_DEVICE, "solver read-back failed");
+  if (rc) return rc;
+  const int* f = w.hflag;
+  if (f[2 * nrhs + F_BAD]) return pg_set_err(c, PG_ERR_NONFINITE, "K_ff has a non-positive or non-finite diagonal entry");
+  if (f[2 * nrhs + F_STUCK]) return pg_set_err(c, PG_ERR_DEVICE, "a grid barrier of the solver ran out");
+  for (int s = 0; s < nrhs; ++s) {
+    const double rr = sc[(size_t)s * S_NSC + S_RELRES];
+    if (iters) iters[s] = f[nrhs + s];
+    if (relres) relres[s] = rr;
+    *all = *all && f[s] && std::isfinite(rr);
+  }
+  return 0;
+}
+
+// ---------------------------------------------------------------- homogenization
+constexpr int kHomBlocks = 2 * 148;
 
 __device__ __forceinline__ void block_sum(double* sh, double v, double* out) {
   sh[threadIdx.x] = v;
@@ -47,336 +760,6 @@ __device__ __forceinline__ void block_sum(double* sh, double v, double* out) {
   if (threadIdx.x == 0) *out = sh[0];
   __syncthreads();
 }
-
-// Rows of block b: [b * chunk, min(n, (b + 1) * chunk)).
-__device__ __forceinline__ void block_rows(int n, int nb, int* r0, int* r1) {
-  const int chunk = (n + nb - 1) / nb;
-  *r0 = min(n, (int)blockIdx.x * chunk);
-  *r1 = min(n, *r0 + chunk);
-}
-
-__global__ void __launch_bounds__(kThreads) k_pcg_diag(const int* rp, const int* ci, const double* val, int n,
-                                                       double* dinv, int* bad) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double d = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k)
-      if (ci[k] == i) d = val[k];
-    if (!(d > 0.0) || !isfinite(d)) { atomicOr(bad, 1); dinv[i] = 0.0; }
-    else dinv[i] = 1.0 / d;
-  }
-}
-
-// (A x)[row] with kRowGroup lanes per row, lane-strided products then a fixed shuffle tree; every
-// lane of the warp calls it (valid = false gives an empty row) so the shuffles stay converged.
-__device__ __forceinline__ double row_dot(const PcgArgs& a, const double* x, int row, bool valid) {
-  const int lane = threadIdx.x % kRowGroup;
-  double v = 0.0;
-  const int k0 = valid ? a.rp[row] : 0, k1 = valid ? a.rp[row + 1] : 0;
-  for (int k = k0 + lane; k < k1; k += kRowGroup) v += a.val[k] * x[a.ci[k]];
-#pragma unroll
-  for (int o = kRowGroup / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, kRowGroup);
-  return v;  // valid in lane 0 of the group
-}
-
-// r = b - A x, z = D^-1 r, p = z; partials of r.z, b.b, r.r
-__global__ void __launch_bounds__(kThreads) k_pcg_start(PcgArgs a, const double* b) {
-  __shared__ double sh[kThreads];
-  int r0, r1;
-  block_rows(a.n, a.nb, &r0, &r1);
-  const int grp = threadIdx.x / kRowGroup, lane = threadIdx.x % kRowGroup, ngrp = kThreads / kRowGroup;
-  for (int s = 0; s < a.nrhs; ++s) {
-    const size_t o = (size_t)s * a.n;
-    double rz = 0.0, bb = 0.0, rr = 0.0;
-    for (int i0 = r0; i0 < r1; i0 += ngrp) {
-      const int i = i0 + grp;
-      const double ax = row_dot(a, a.x + o, i, i < r1);
-      if (i < r1 && lane == 0) {
-        const double ri = b[o + i] - ax;
-        const double zi = a.dinv[i] * ri;
-        a.r[o + i] = ri; a.z[o + i] = zi; a.p[(size_t)i * a.nrhs + s] = zi;
-        rz += ri * zi; bb += b[o + i] * b[o + i]; rr += ri * ri;
-      }
-    }
-    block_sum(sh, rz, &a.part[(0 * a.nrhs + s) * a.nb + blockIdx.x]);
-    block_sum(sh, bb, &a.part[(1 * a.nrhs + s) * a.nb + blockIdx.x]);
-    block_sum(sh, rr, &a.part[(2 * a.nrhs + s) * a.nb + blockIdx.x]);
-  }
-}
-
-// one block per right-hand side: ordered sums of the partials
-__global__ void __launch_bounds__(kThreads) k_pcg_start_reduce(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  const int s = blockIdx.x;
-  double v[3];
-  for (int k = 0; k < 3; ++k) {
-    double t = 0.0;
-    for (int i = threadIdx.x; i < a.nb; i += kThreads) t += a.part[(k * a.nrhs + s) * a.nb + i];
-    block_sum(sh, t, &sh[0]);  // result lands in sh[0] after the call's last sync
-    v[k] = sh[0];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double* sc = a.sc + s * S_NSC;
-    sc[S_RZ] = v[0]; sc[S_BB] = v[1]; sc[S_RR] = v[2];
-    const double nb = sqrt(v[1]);
-    sc[S_RELRES] = nb > 0.0 ? sqrt(v[2]) / nb : 0.0;
-    const int done = (nb == 0.0) || (sc[S_RELRES] <= a.rtol);
-    a.flag[s] = done;
-    a.flag[a.nrhs + s] = 0;
-    if (done) atomicSub(&a.flag[2 * a.nrhs], 1);
-  }
-}
-
-// q = A p; partials of p.q.  The right-hand sides still iterating share one pass over the matrix
-// (up to kSpmvRhs at a time): each row's values and column indices are read once and multiplied
-// with every right-hand side's p, whose values for one column are adjacent (p is interleaved by
-// right-hand side).  Each right-hand side's sums are the ones row_dot forms (same lane-strided
-// products, same shuffle tree), so its iterates do not depend on the others.
-constexpr int kSpmvRhs = 8;
-__global__ void __launch_bounds__(kThreads) k_pcg_spmv(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  if (a.flag[2 * a.nrhs] == 0) return;
-  int r0, r1;
-  block_rows(a.n, a.nb, &r0, &r1);
-  const int grp = threadIdx.x / kRowGroup, lane = threadIdx.x % kRowGroup, ngrp = kThreads / kRowGroup;
-  for (int s0 = 0; s0 < a.nrhs; s0 += kSpmvRhs) {
-    const int ns = min(kSpmvRhs, a.nrhs - s0);
-    bool act[kSpmvRhs];
-    double pq[kSpmvRhs];
-#pragma unroll
-    for (int j = 0; j < kSpmvRhs; ++j) { act[j] = j < ns && !a.flag[s0 + j]; pq[j] = 0.0; }
-    for (int i0 = r0; i0 < r1; i0 += ngrp) {
-      const int i = i0 + grp;
-      const bool valid = i < r1;
-      double v[kSpmvRhs];
-#pragma unroll
-      for (int j = 0; j < kSpmvRhs; ++j) v[j] = 0.0;
-      const int k0 = valid ? a.rp[i] : 0, k1 = valid ? a.rp[i + 1] : 0;
-      for (int k = k0 + lane; k < k1; k += kRowGroup) {
-        const double av = a.val[k];
-        const int c = a.ci[k];
-#pragma unroll
-        for (int j = 0; j < kSpmvRhs; ++j)
-          if (act[j]) v[j] += av * a.p[(size_t)c * a.nrhs + s0 + j];
-      }
-#pragma unroll
-      for (int j = 0; j < kSpmvRhs; ++j) {
-        if (!act[j]) continue;   // uniform over the block
-#pragma unroll
-        for (int o = kRowGroup / 2; o > 0; o >>= 1) v[j] += __shfl_down_sync(0xffffffffu, v[j], o, kRowGroup);
-        if (valid && lane == 0) {
-          a.q[(size_t)(s0 + j) * a.n + i] = v[j];
-          pq[j] += a.p[(size_t)i * a.nrhs + s0 + j] * v[j];
-        }
-      }
-    }
-    for (int j = 0; j < ns; ++j)
-      if (act[j]) block_sum(sh, pq[j], &a.part[(0 * a.nrhs + s0 + j) * a.nb + blockIdx.x]);
-  }
-}
-
-// The same product for exactly NS right-hand sides (NS = nrhs <= 8, known at compile time): a
-// column's NS values of p are read as 16-byte pairs when NS is even, and every lane keeps two
-// nonzeros in flight; each right-hand side's products are still added in the lane's nonzero
-// order, so the sums are those of k_pcg_spmv.
-template <int NS>
-__device__ __forceinline__ void load_p(const double* __restrict__ p, int c, double* out) {
-  if constexpr (NS % 2 == 0) {
-    const double2* q = reinterpret_cast<const double2*>(p + (size_t)c * NS);
-#pragma unroll
-    for (int j = 0; j < NS / 2; ++j) { const double2 t = __ldg(q + j); out[2 * j] = t.x; out[2 * j + 1] = t.y; }
-  } else {
-#pragma unroll
-    for (int j = 0; j < NS; ++j) out[j] = __ldg(p + (size_t)c * NS + j);
-  }
-}
-
-template <int NS>
-__global__ void __launch_bounds__(kThreads) k_pcg_spmv_n(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  if (a.flag[2 * a.nrhs] == 0) return;
-  int r0, r1;
-  block_rows(a.n, a.nb, &r0, &r1);
-  const int grp = threadIdx.x / kRowGroup, lane = threadIdx.x % kRowGroup, ngrp = kThreads / kRowGroup;
-  bool act[NS];
-  double pq[NS];
-#pragma unroll
-  for (int j = 0; j < NS; ++j) { act[j] = !a.flag[j]; pq[j] = 0.0; }
-  for (int i0 = r0; i0 < r1; i0 += ngrp) {
-    const int i = i0 + grp;
-    const bool valid = i < r1;
-    double v[NS];
-#pragma unroll
-    for (int j = 0; j < NS; ++j) v[j] = 0.0;
-    const int k0 = valid ? a.rp[i] : 0, k1 = valid ? a.rp[i + 1] : 0;
-    int k = k0 + lane;
-    for (; k + kRowGroup < k1; k += 2 * kRowGroup) {
-      const double av0 = __ldg(a.val + k), av1 = __ldg(a.val + k + kRowGroup);
-      const int c0 = __ldg(a.ci + k), c1 = __ldg(a.ci + k + kRowGroup);
-      double p0[NS], p1[NS];
-      load_p<NS>(a.p, c0, p0);
-      load_p<NS>(a.p, c1, p1);
-#pragma unroll
-      for (int j = 0; j < NS; ++j) v[j] += av0 * p0[j];
-#pragma unroll
-      for (int j = 0; j < NS; ++j) v[j] += av1 * p1[j];
-    }
-    if (k < k1) {
-      const double av0 = __ldg(a.val + k);
-      double p0[NS];
-      load_p<NS>(a.p, __ldg(a.ci + k), p0);
-#pragma unroll
-      for (int j = 0; j < NS; ++j) v[j] += av0 * p0[j];
-    }
-#pragma unroll
-    for (int j = 0; j < NS; ++j) {
-      if (!act[j]) continue;   // uniform over the block
-#pragma unroll
-      for (int o = kRowGroup / 2; o > 0; o >>= 1) v[j] += __shfl_down_sync(0xffffffffu, v[j], o, kRowGroup);
-      if (valid && lane == 0) {
-        a.q[(size_t)j * a.n + i] = v[j];
-        pq[j] += a.p[(size_t)i * NS + j] * v[j];
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NS; ++j)
-    if (act[j]) block_sum(sh, pq[j], &a.part[(0 * a.nrhs + j) * a.nb + blockIdx.x]);
-}
-
-__global__ void __launch_bounds__(kThreads) k_pcg_alpha(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  if (a.flag[2 * a.nrhs] == 0) return;
-  const int s = blockIdx.x;
-  if (a.flag[s]) return;
-  double t = 0.0;
-  for (int i = threadIdx.x; i < a.nb; i += kThreads) t += a.part[(0 * a.nrhs + s) * a.nb + i];
-  block_sum(sh, t, &sh[0]);
-  if (threadIdx.x == 0) {
-    double* sc = a.sc + s * S_NSC;
-    sc[S_PQ] = sh[0];
-    sc[S_ALPHA] = sc[S_RZ] / sh[0];
-  }
-}
-
-// x += alpha p, r -= alpha q, z = D^-1 r; partials of r.z and r.r
-__global__ void __launch_bounds__(kThreads) k_pcg_update(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  if (a.flag[2 * a.nrhs] == 0) return;
-  int r0, r1;
-  block_rows(a.n, a.nb, &r0, &r1);
-  for (int s = 0; s < a.nrhs; ++s) {
-    if (a.flag[s]) continue;
-    const size_t o = (size_t)s * a.n;
-    const double al = a.sc[s * S_NSC + S_ALPHA];
-    double rz = 0.0, rr = 0.0;
-    for (int i = r0 + threadIdx.x; i < r1; i += kThreads) {
-      a.x[o + i] += al * a.p[(size_t)i * a.nrhs + s];
-      const double ri = a.r[o + i] - al * a.q[o + i];
-      const double zi = a.dinv[i] * ri;
-      a.r[o + i] = ri; a.z[o + i] = zi;
-      rz += ri * zi; rr += ri * ri;
-    }
-    block_sum(sh, rz, &a.part[(1 * a.nrhs + s) * a.nb + blockIdx.x]);
-    block_sum(sh, rr, &a.part[(2 * a.nrhs + s) * a.nb + blockIdx.x]);
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_pcg_beta(PcgArgs a) {
-  __shared__ double sh[kThreads];
-  if (a.flag[2 * a.nrhs] == 0) return;
-  const int s = blockIdx.x;
-  if (a.flag[s]) return;
-  double v[2];
-  for (int k = 0; k < 2; ++k) {
-    double t = 0.0;
-    for (int i = threadIdx.x; i < a.nb; i += kThreads) t += a.part[((1 + k) * a.nrhs + s) * a.nb + i];
-    block_sum(sh, t, &sh[0]);
-    v[k] = sh[0];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double* sc = a.sc + s * S_NSC;
-    sc[S_BETA] = v[0] / sc[S_RZ];
-    sc[S_RZ] = v[0];
-    sc[S_RR] = v[1];
-    sc[S_RELRES] = sqrt(v[1]) / sqrt(sc[S_BB]);
-    a.flag[a.nrhs + s] += 1;
-    if (sc[S_RELRES] <= a.rtol || !isfinite(sc[S_RELRES])) {
-      a.flag[s] = 1;
-      atomicSub(&a.flag[2 * a.nrhs], 1);
-    }
-  }
-}
-
-// p = z + beta p for the right-hand sides still iterating
-__global__ void __launch_bounds__(kThreads) k_pcg_dir(PcgArgs a) {
-  if (a.flag[2 * a.nrhs] == 0) return;
-  int r0, r1;
-  block_rows(a.n, a.nb, &r0, &r1);
-  for (int s = 0; s < a.nrhs; ++s) {
-    if (a.flag[s]) continue;
-    const size_t o = (size_t)s * a.n;
-    const double be = a.sc[s * S_NSC + S_BETA];
-    for (int i = r0 + threadIdx.x; i < r1; i += kThreads) {
-      double& pi = a.p[(size_t)i * a.nrhs + s];
-      pi = a.z[o + i] + be * pi;
-    }
-  }
-}
-
-void launch_iteration(const PcgArgs& a, cudaStream_t st) {
-  switch (a.nrhs) {
-    case 1: k_pcg_spmv_n<1><<<a.nb, kThreads, 0, st>>>(a); break;
-    case 2: k_pcg_spmv_n<2><<<a.nb, kThreads, 0, st>>>(a); break;
-    case 3: k_pcg_spmv_n<3><<<a.nb, kThreads, 0, st>>>(a); break;
-    case 4: k_pcg_spmv_n<4><<<a.nb, kThreads, 0, st>>>(a); break;
-    case 6: k_pcg_spmv_n<6><<<a.nb, kThreads, 0, st>>>(a); break;
-    default: k_pcg_spmv<<<a.nb, kThreads, 0, st>>>(a); break;
-  }
-  k_pcg_alpha<<<a.nrhs, kThreads, 0, st>>>(a);
-  k_pcg_update<<<a.nb, kThreads, 0, st>>>(a);
-  k_pcg_beta<<<a.nrhs, kThreads, 0, st>>>(a);
-  k_pcg_dir<<<a.nb, kThreads, 0, st>>>(a);
-}
-
-int pcg_reserve(pg_ctx* c, int nrhs) {
-  PcgWork& w = c->pcg;
-  const int n = c->s.n_free;
-  if (w.cap_rhs >= nrhs && w.n == n) return 0;
-  if (!w.stream) {
-    if (cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&w.ev, cudaEventDisableTiming) != cudaSuccess)
-      return pg_set_err(c, PG_ERR_DEVICE, "solver stream creation failed");
-    if (cudaMallocHost(&w.hflag, sizeof(int) * 64) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "pinned flag allocation failed");
-  }
-  w.n = n;
-  w.cap_rhs = nrhs;
-  w.nb = 8 * 148;   // row ranges: enough blocks in flight to hide the matrix-vector latency
-  int rc = 0;
-  if (!w.dinv) rc |= pg_dalloc(c, (size_t)n, &w.dinv);
-  if (!w.ci) {
-    // column indices of K_ff (the assembly writes values by slot and never needs them)
-    int* ci = nullptr;
-    rc |= pg_dalloc(c, c->s.ci[0].size(), &ci);
-    if (!rc && !c->s.ci[0].empty() &&
-        cudaMemcpyAsync(ci, c->s.ci[0].data(), c->s.ci[0].size() * sizeof(int), cudaMemcpyHostToDevice, c->up) != cudaSuccess)
-      rc = 1;
-    w.ci = ci;
-  }
-  rc |= pg_dalloc(c, (size_t)n * nrhs, &w.r);
-  rc |= pg_dalloc(c, (size_t)n * nrhs, &w.z);
-  rc |= pg_dalloc(c, (size_t)n * nrhs, &w.p);
-  rc |= pg_dalloc(c, (size_t)n * nrhs, &w.q);
-  rc |= pg_dalloc(c, (size_t)3 * nrhs * w.nb, &w.part);
-  rc |= pg_dalloc(c, (size_t)S_NSC * nrhs, &w.sc);
-  rc |= pg_dalloc(c, (size_t)2 * nrhs + 1, &w.flag);
-  if (rc) return PG_ERR_DEVICE;
-  return pg_alloc_sync(c);
-}
-
-// ---------------------------------------------------------------- homogenization
-constexpr int kHomBlocks = 2 * 148;
 
 // Per block: sum over a fixed element range of w * sigma (NV entries) and w.
 template <int DIM>
@@ -487,61 +870,21 @@ int pg_pcg_solve(pg_ctx* c, const double* d_b, double* d_x, int nrhs, double rto
   if (!pg_resident(c)) return pg_set_err(c, PG_ERR_STATE, "the context has no device residency (pg_upload it first)");
   if (!c->assembled) return pg_set_err(c, PG_ERR_STATE, "assemble K before solving with it");
   if (c->s.n_free == 0) return pg_set_err(c, PG_ERR_STATE, "no free degrees of freedom");
-  if (int rc = pcg_reserve(c, nrhs)) return rc;
+  if (int rc = pcg_reserve(c, std::min(nrhs, kMaxRhs))) return rc;
   PcgWork& w = c->pcg;
-  const int n = c->s.n_free;
   // order after the assembly on the context's stream
   cudaEventRecord(w.ev, c->stream);
   cudaStreamWaitEvent(w.stream, w.ev, 0);
-  PcgArgs a{c->P.rp[0], w.ci, c->P.val[0], n, nrhs, w.nb, rtol,
-            w.dinv, d_x, w.r, w.z, w.p, w.q, w.part, w.sc, w.flag};
-  // the diagonal changes with every assembly: recompute it
-  cudaMemsetAsync(w.flag, 0, sizeof(int) * (2 * nrhs + 1), w.stream);
-  k_pcg_diag<<<2 * 148, kThreads, 0, w.stream>>>(a.rp, a.ci, a.val, n, w.dinv, w.flag + 2 * nrhs);
-  cudaMemcpyAsync(w.hflag, w.flag + 2 * nrhs, sizeof(int), cudaMemcpyDeviceToHost, w.stream);
-  if (cudaStreamSynchronize(w.stream) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "solver set-up failed");
-  if (w.hflag[0]) return pg_set_err(c, PG_ERR_NONFINITE, "K_ff has a non-positive or non-finite diagonal entry");
-  const int active = nrhs;
-  cudaMemcpyAsync(w.flag + 2 * nrhs, &active, sizeof(int), cudaMemcpyHostToDevice, w.stream);
-  k_pcg_start<<<w.nb, kThreads, 0, w.stream>>>(a, d_b);
-  k_pcg_start_reduce<<<nrhs, kThreads, 0, w.stream>>>(a);
-  // capture kChunk iterations once, replay until every right-hand side is done or max_it
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  if (cudaStreamBeginCapture(w.stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-    return pg_set_err(c, PG_ERR_DEVICE, "graph capture failed to start");
-  for (int it = 0; it < kChunk; ++it) launch_iteration(a, w.stream);
-  if (cudaStreamEndCapture(w.stream, &graph) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    return pg_set_err(c, PG_ERR_DEVICE, "graph instantiation failed");
+  bool all = true;
+  for (int s = 0; s < nrhs; s += kMaxRhs) {
+    const size_t o = (size_t)s * c->s.n_free;
+    if (int rc = pcg_pass(c, d_b + o, d_x + o, std::min(kMaxRhs, nrhs - s), rtol, max_it, iters ? iters + s : nullptr,
+                          relres ? relres + s : nullptr, &all))
+      return rc;
   }
-  int done_iters = 0;
-  int rc = 0;
-  while (true) {
-    cudaMemcpyAsync(w.hflag, w.flag + 2 * nrhs, sizeof(int), cudaMemcpyDeviceToHost, w.stream);
-    if (cudaStreamSynchronize(w.stream) != cudaSuccess) { rc = pg_set_err(c, PG_ERR_DEVICE, "solver iteration failed"); break; }
-    if (w.hflag[0] == 0 || done_iters >= max_it) break;
-    cudaGraphLaunch(exec, w.stream);
-    done_iters += kChunk;
-  }
-  cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
-  if (rc) return rc;
-  // results
-  std::vector<int> fl(2 * nrhs + 1);
-  std::vector<double> sc((size_t)S_NSC * nrhs);
-  cudaMemcpyAsync(fl.data(), w.flag, sizeof(int) * fl.size(), cudaMemcpyDeviceToHost, w.stream);
-  cudaMemcpyAsync(sc.data(), w.sc, sizeof(double) * sc.size(), cudaMemcpyDeviceToHost, w.stream);
-  if (cudaStreamSynchronize(w.stream) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "solver read-back failed");
   // later work on the context's stream sees the solution
   cudaEventRecord(w.ev, w.stream);
   cudaStreamWaitEvent(c->stream, w.ev, 0);
-  bool all = true;
-  for (int s = 0; s < nrhs; ++s) {
-    if (iters) iters[s] = fl[nrhs + s];
-    if (relres) relres[s] = sc[(size_t)s * S_NSC + S_RELRES];
-    all = all && fl[s] && std::isfinite(sc[(size_t)s * S_NSC + S_RELRES]);
-  }
   if (!all) return pg_set_err(c, PG_ERR_STATE, "PCG did not reach the tolerance within max_it");
   return 0;
 }
