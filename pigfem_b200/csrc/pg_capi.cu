@@ -6,7 +6,6 @@
 // host arrays; pointers are never retained across calls.
 #include "pg_ctx.h"
 #include "pg_launch.cuh"
-#include "pg_tile.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -61,18 +60,76 @@ __global__ void k_sum_final(const double* part, int n, double* out) {
   }
 }
 
+// The structured rows' constants (pg_rows.cuh): the shapes' element matrices (k_shape_consts) summed
+// over a node's adjacent elements in adjacency order, per class and material.
+template <class S, int DIM>
+void class_rows(int npe, int cls, int m, const std::vector<double>& shapes, bool f32, double* rows, double* g) {
+  const int nd = npe * DIM, nv = DIM == 2 ? 3 : 6;
+  for (int i = 0; i < DIM * S::NN * DIM; ++i) rows[i] = 0.0;
+  for (int i = 0; g && i < DIM * nv; ++i) g[i] = 0.0;
+  for (int a = 0; a < S::NADJ; ++a) {
+    const int sub = S::ent(a, 3), la = S::ent(a, 4);
+    const int sh = (DIM == 3 || npe == 4) ? sub : 2 * ((cls + S::ent(a, 0) + S::ent(a, 1)) & 1) + sub;
+    const double* ke = shapes.data() + (size_t)(sh * 3 + m) * pgd::shape_doubles(DIM, npe);
+    const double* gm = ke + 2 * nd * nd;
+    if (f32) ke += nd * nd;
+    for (int q = 0; q < DIM; ++q) {
+      for (int lb = 0; lb < npe; ++lb)
+        for (int d = 0; d < DIM; ++d)
+          rows[(q * S::NN + S::ent(a, 5 + lb)) * DIM + d] += ke[(la * DIM + q) * nd + lb * DIM + d];
+      for (int v = 0; g && v < nv; ++v) g[q * nv + v] += gm[(la * DIM + q) * nv + v];
+    }
+  }
+}
+int structured_constants(pg_ctx* c) {
+  const pg::Setup& s = c->s;
+  const int dim = s.dim, npe = s.npe, nv = dim == 2 ? 3 : 6, nc = dim == 2 ? 2 : 1;
+  std::vector<double> shapes((size_t)pgd::shape_count(dim, npe) * 3 * pgd::shape_doubles(dim, npe));
+  if ((dim == 2 ? pgl::shape_consts<2>(c, c->P, shapes.data()) : pgl::shape_consts<3>(c, c->P, shapes.data())) != 0)
+    return set_err(c, PG_ERR_DEVICE, "structured-row constants failed");
+  const int per = pgd::pattern_period(dim, npe), nr = pgd::row_coefs(dim);
+  std::vector<double> pat((size_t)2 * 3 * 2 * per), srow((size_t)3 * nc * nr, 0.0), sg((size_t)3 * nc * dim * nv, 0.0);
+  for (int prec = 0; prec < 2; ++prec)
+    for (int m = 0; m < 3; ++m) {
+      double rows[2][135];
+      double* g = prec == 0 ? sg.data() + (size_t)m * nc * dim * nv : nullptr;
+      int len[2] = {0, 0};
+      if (dim == 3) {
+        class_rows<pgd::Tet4Stencil0, 3>(4, 0, m, shapes, prec == 1, rows[0], g);
+        class_rows<pgd::Tet4Stencil0, 3>(4, 0, m, shapes, prec == 1, rows[1], nullptr);
+        len[0] = len[1] = 135;
+      } else if (npe == 4) {
+        class_rows<pgd::Quad4Stencil0, 2>(4, 0, m, shapes, prec == 1, rows[0], g);
+        len[0] = 36;
+      } else {
+        class_rows<pgd::Tri3Stencil0, 2>(3, 0, m, shapes, prec == 1, rows[0], g);
+        class_rows<pgd::Tri3Stencil1, 2>(3, 1, m, shapes, prec == 1, rows[1], g ? g + dim * nv : nullptr);
+        len[0] = 36;
+        len[1] = 20;
+      }
+      if (prec == 0)
+        for (int cls = 0; cls < nc; ++cls) std::copy(rows[cls], rows[cls] + len[cls], srow.begin() + (size_t)(m * nc + cls) * nr);
+      std::vector<double> p(rows[0], rows[0] + len[0]);
+      p.insert(p.end(), rows[1], rows[1] + len[1]);
+      for (int odd = 0; odd < 2; ++odd)
+        for (int i = 0; i < per; ++i) pat[((size_t)(prec * 3 + m) * 2 + odd) * per + i] = p[(i + odd) % per];
+    }
+  PG_TRY(upload(c, pat, &c->P.pat));
+  PG_TRY(upload(c, srow, &c->P.srow));
+  PG_TRY(upload(c, sg, &c->P.sg));
+  return 0;
+}
+
 int launch(pg_ctx* c, double t_frac, int flags) {
-  if (!c->ev[0])
-    for (int i = 0; i < 6; ++i) cudaEventCreateWithFlags(&c->ev[i], cudaEventDefault);
+  if (c->timing && !c->ev[0])
+    for (int i = 0; i < 5; ++i) cudaEventCreateWithFlags(&c->ev[i], cudaEventDefault);
   pgd::DevProblem P = c->P;
   P.U = c->d_U;
   P.flags = flags;
   for (int v = 0; v < 6; ++v) P.eps_macro[v] = c->s.desc.eps_macro[v] * t_frac;
   const int dim = c->s.dim;
-  const bool fp32 = (flags & PG_FP32) != 0;
-  const bool jac = (flags & PG_JAC) != 0;   // without it: the residual-only kernels
-  if (dim == 2) pgl::assembly<2>(c, P, jac, fp32);
-  else pgl::assembly<3>(c, P, jac, fp32);
+  if (dim == 2) pgl::assembly<2>(c, P);
+  else pgl::assembly<3>(c, P);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(c, PG_ERR_DEVICE, std::string("launch failed: ") + cudaGetErrorString(e));
   return 0;
@@ -175,231 +232,131 @@ int pg_upload(pg_ctx* c) {
     const int na = s.dn_node[a];
     for (int q = 0; q < dim; ++q) if (s.node_dof[(size_t)na * dim + q] < s.n_free) mask[a] |= (uint8_t)(1 << q);
   }
-  // neighbour masks, adjacency slots, fast/general split
+  // neighbour masks, adjacency slots
   std::vector<uint8_t> nbr_mask(s.dn_nbr.size());
   for (size_t k = 0; k < s.dn_nbr.size(); ++k) nbr_mask[k] = mask[s.dn_nbr[k]];
-  std::vector<int> slot32(s.dn_adj.size(), 0), slot_off(s.dn_adj.size() + 1, 0);
+  std::vector<int> slot32(s.dn_adj.size(), 0), slot_off(s.dn_adj.size(), 0);
   std::vector<uint8_t> slots;
-  const int maxnb = (dim == 2) ? 9 : 15;
-  std::vector<int> fast, slow;
-  int maxnb_general = 1;
   for (int a = 0; a < s.n_dn; ++a) {
     const int* nb = s.dn_nbr.data() + s.dn_nbr_off[a];
     const int nn = s.dn_nbr_off[a + 1] - s.dn_nbr_off[a];
     if (nn > 255) return set_err(c, PG_ERR_UNSUPPORTED, "a DOF node with more than 255 neighbours");
-    bool ok = nn <= maxnb;
     for (int k = s.dn_adj_off[a]; k < s.dn_adj_off[a + 1]; ++k) {
-      const int e = s.dn_adj[k] >> 5;
-      std::vector<int> en;
-      if (s.cut_of[e] < 0) { ok = ok && true; for (int q = 0; q < s.npe; ++q) en.push_back(s.conn[(size_t)e * s.npe + q]); }
-      else {
-        ok = false;
-        const int cc = s.cut_of[e];
-        for (int q = s.cut_node_off[cc]; q < s.cut_node_off[cc + 1]; ++q) en.push_back(s.cut_nodes[q]);
-      }
+      const int e = s.dn_adj[k] >> 5, cc = s.cut_of[e];
+      const int* en = cc < 0 ? &s.conn[(size_t)e * s.npe] : &s.cut_nodes[s.cut_node_off[cc]];
+      const int mn = cc < 0 ? s.npe : s.cut_node_off[cc + 1] - s.cut_node_off[cc];
+      int pos[pgd::kMaxNodesCut];
+      if (mn > pgd::kMaxNodesCut) return set_err(c, PG_ERR_UNSUPPORTED, "a cut element with more than 32 nodes");
       slot_off[k] = (int)slots.size();
-      const size_t first_slot = slots.size();
-      for (size_t lb = 0; lb < en.size(); ++lb) {
+      for (int lb = 0; lb < mn; ++lb) {
         const int db = s.node_dn[en[lb]];
-        const int pos = (int)(std::lower_bound(nb, nb + nn, db) - nb);
-        if (pos >= nn || nb[pos] != db) return set_err(c, PG_ERR_STATE, "internal: adjacency without neighbour slot");
-        // the lanes of a row group add an element's blocks concurrently: its nodes need distinct slots
-        for (size_t k2 = first_slot; k2 < slots.size(); ++k2)
-          if (slots[k2] == pos) return set_err(c, PG_ERR_UNSUPPORTED, "an element holds a node and its periodic image");
-        slots.push_back((uint8_t)pos);
-        if (s.cut_of[e] < 0) slot32[k] |= pos << (8 * lb);
+        pos[lb] = (int)(std::lower_bound(nb, nb + nn, db) - nb);
+        if (pos[lb] >= nn || nb[pos[lb]] != db) return set_err(c, PG_ERR_STATE, "internal: adjacency without neighbour slot");
+        // an element's nodes need distinct slots
+        for (int k2 = 0; k2 < lb; ++k2)
+          if (pos[k2] == pos[lb]) return set_err(c, PG_ERR_UNSUPPORTED, "an element holds a node and its periodic image");
+        if (cc < 0) slot32[k] |= pos[lb] << (8 * lb);
+        else slots.push_back((uint8_t)pos[lb]);
       }
     }
-    slot_off[s.dn_adj.size()] = (int)slots.size();
-    (void)ok;
-    slow.push_back(a);
-    maxnb_general = std::max(maxnb_general, nn);
   }
-  slot_off[s.dn_adj.size()] = (int)slots.size();
-  // Structured-grid stencil nodes (pg_stencil.cuh): interior DOF nodes two cells from the domain
-  // boundary whose adjacency, neighbours and row layout match their class table exactly, whose
-  // elements are all uncut and whose neighbour DOFs are all free.  Everything else is general.
-  std::vector<int4> stencil;
+  // Structured rows (pg_rows.cuh): DOF nodes inside the grid whose adjacency, neighbours and row
+  // layout match their class table exactly, whose elements are all uncut and of one material and
+  // whose neighbour DOFs are all free.  Everything else is general.
+  std::vector<int4> stencil;   // {node id, first DOF, first CSR value, class | material << 4}
+  std::vector<int4> chunks;
+  std::vector<int> fast, slow;
   {
     const int Nx = s.desc.n[0], Ny = s.desc.n[1], Nz = (dim == 3) ? s.desc.n[2] : 0;
     const int sx = Nx + 1, sxy = sx * (Ny + 1);
-    const bool grid_ok = (s.etype == pg::TRI3 || s.etype == pg::TET4);
+    const bool quad = s.etype == pg::QUAD4;
+    const int per_cell = dim == 3 ? 6 : (quad ? 1 : 2);
     std::vector<char> in_stencil(s.n_dn, 0);
-    std::vector<std::vector<int4>> by_class(2);
-    for (int a = 0; a < s.n_dn && grid_ok; ++a) {
+    std::vector<int4> by_node;
+    int open_next = -1, open_cls = -1;   // the CSR value and class that continue the open chunk
+    const int phase_of[2] = {0, 2 * pgd::Tri3Stencil0::NN * 2};
+    for (int a = 0; a < s.n_dn; ++a) {
       const int nid = s.dn_node[a];
       if (nid >= s.n_std) continue;
       const int i = nid % sx, j = (nid / sx) % (Ny + 1), k = nid / sxy;
-      if (i < 2 || i > Nx - 2 || j < 2 || j > Ny - 2) continue;
-      if (dim == 3 && (k < 2 || k > Nz - 2)) continue;
-      const int cls = (dim == 2) ? ((i + j) % 2) : 0;
-      const int NN = (dim == 2) ? (cls == 0 ? pgd::Tri3Stencil0::NN : pgd::Tri3Stencil1::NN) : pgd::Tet4Stencil0::NN;
-      const int NADJ = (dim == 2) ? (cls == 0 ? pgd::Tri3Stencil0::NADJ : pgd::Tri3Stencil1::NADJ) : pgd::Tet4Stencil0::NADJ;
+      if (i < 1 || i > Nx - 1 || j < 1 || j > Ny - 1) continue;
+      if (dim == 3 && (k < 1 || k > Nz - 1)) continue;
+      const int cls = (dim == 2 && !quad) ? ((i + j) % 2) : 0;
+      const int NN = dim == 3 ? pgd::Tet4Stencil0::NN : (cls == 0 ? pgd::Tri3Stencil0::NN : pgd::Tri3Stencil1::NN);
+      const int NADJ = dim == 3 ? pgd::Tet4Stencil0::NADJ
+                                : (quad ? pgd::Quad4Stencil0::NADJ : (cls == 0 ? pgd::Tri3Stencil0::NADJ : pgd::Tri3Stencil1::NADJ));
       auto off = [&](int q, int d) {
-        return (dim == 2) ? (cls == 0 ? pgd::Tri3Stencil0::off(q, d) : pgd::Tri3Stencil1::off(q, d)) : pgd::Tet4Stencil0::off(q, d);
+        return dim == 3 ? pgd::Tet4Stencil0::off(q, d) : (cls == 0 ? pgd::Tri3Stencil0::off(q, d) : pgd::Tri3Stencil1::off(q, d));
       };
       auto entv = [&](int q, int cidx) {
-        return (dim == 2) ? (cls == 0 ? pgd::Tri3Stencil0::ent(q, cidx) : pgd::Tri3Stencil1::ent(q, cidx)) : pgd::Tet4Stencil0::ent(q, cidx);
+        if (dim == 3) return pgd::Tet4Stencil0::ent(q, cidx);
+        if (quad) return pgd::Quad4Stencil0::ent(q, cidx);
+        return cls == 0 ? pgd::Tri3Stencil0::ent(q, cidx) : pgd::Tri3Stencil1::ent(q, cidx);
       };
       bool ok = (s.dn_nbr_off[a + 1] - s.dn_nbr_off[a]) == NN && (s.dn_adj_off[a + 1] - s.dn_adj_off[a]) == NADJ;
       for (int q = 0; ok && q < NN; ++q) {
         const int nb = s.dn_node[s.dn_nbr[s.dn_nbr_off[a] + q]];
         ok = nb == nid + off(q, 0) + off(q, 1) * sx + off(q, 2) * sxy && mask[s.dn_nbr[s.dn_nbr_off[a] + q]] == (1 << dim) - 1;
       }
+      int mat = -1;
       for (int q = 0; ok && q < NADJ; ++q) {
         const int ci = i + entv(q, 0), cj = j + entv(q, 1), ck = k + entv(q, 2);
-        const int e = (dim == 2) ? 2 * (cj * Nx + ci) + entv(q, 3) : 6 * ((ck * Ny + cj) * Nx + ci) + entv(q, 3);
+        const int e = per_cell * ((ck * Ny + cj) * Nx + ci) + entv(q, 3);
         const int entry = s.dn_adj[s.dn_adj_off[a] + q];
         ok = (entry >> 5) == e && (entry & 31) == entv(q, 4) && s.cut_of[e] < 0;
-        for (int n = 0; ok && n <= dim; ++n) {
+        if (ok && mat < 0) mat = s.elem_mat[e];
+        ok = ok && s.elem_mat[e] == mat;
+        for (int n = 0; ok && n < s.npe; ++n) {
           const int sl = entv(q, 5 + n);
-          ok = s.conn[(size_t)e * (dim + 1) + n] == nid + off(sl, 0) + off(sl, 1) * sx + off(sl, 2) * sxy;
+          ok = s.conn[(size_t)e * s.npe + n] == nid + off(sl, 0) + off(sl, 1) * sx + off(sl, 2) * sxy;
         }
       }
       if (!ok) continue;
       const int g0 = s.node_dof[(size_t)nid * dim];
       for (int q = 0; ok && q < dim; ++q) ok = s.node_dof[(size_t)nid * dim + q] == g0 + q && g0 + q < s.n_free;
       if (!ok) continue;
-      const int row0 = s.rp[0][g0];
+      const int row0 = s.rp[0][g0], len = dim * NN * dim;
       for (int q = 0; ok && q < dim; ++q)
         ok = s.rp[0][g0 + q] == row0 + q * NN * dim && s.rp[0][g0 + q + 1] - s.rp[0][g0 + q] == NN * dim &&
              s.rp[1][g0 + q + 1] == s.rp[1][g0 + q];
       if (!ok) continue;
-      by_class[cls].push_back(make_int4(nid, g0, row0, cls));
       in_stencil[a] = 1;
+      by_node.push_back(make_int4(nid, g0, row0, cls | (mat << 4)));
+      // the FP32-mixed rows are those two cells from the boundary; the ring next to it stays FP64
+      const bool ring = i < 2 || i > Nx - 2 || j < 2 || j > Ny - 2 || (dim == 3 && (k < 2 || k > Nz - 2));
+      const int kind = mat | (ring ? 4 : 0);
+      if (!chunks.empty() && open_next == row0 && chunks.back().w == kind && chunks.back().y + len <= pgd::kChunkValues &&
+          (dim == 3 || quad || open_cls != cls)) {
+        chunks.back().y += len;
+      } else {
+        chunks.push_back(make_int4(row0, len, (dim == 2 && !quad) ? phase_of[cls] : 0, kind));
+      }
+      open_next = row0 + len;
+      open_cls = cls;
     }
-    // each class segment padded to whole warps (entries with node -1): a warp's nodes then share
-    // one class and one row length, which the staged row stores of the 2D kernel rely on
+    // the residual's nodes by class (each padded to whole warps with node -1), so that a warp's
+    // nodes share a class
     for (int cls = 0; cls < 2; ++cls) {
-      auto& v = by_class[cls];
-      if (v.empty()) continue;
-      stencil.insert(stencil.end(), v.begin(), v.end());
+      for (const int4& v : by_node) if ((v.w & 15) == cls) stencil.push_back(v);
       while (stencil.size() % 32) stencil.push_back(make_int4(-1, 0, 0, cls));
     }
-    // 2D tiles of 16 x 8 grid nodes (pg_tile.cuh): per tile 64 class-0 then 64 class-1 node
-    // entries in row-major order, each with its run's offset in the tile's stage (a tile row of
-    // nodes is 8 runs of 36 and 8 of 20 values), and the contiguous CSR segments of each tile row
-    if (dim == 2 && grid_ok) {
-      std::vector<int4> st_of(s.n_std, make_int4(-1, 0, 0, 0));
-      for (int cls = 0; cls < 2; ++cls)
-        for (const int4& v : by_class[cls]) st_of[v.x] = v;
-      const int runlen[2] = {2 * pgd::Tri3Stencil0::NN * 2, 2 * pgd::Tri3Stencil1::NN * 2};
-      std::vector<int4> tiles, tnodes, segs;
-      for (int j0 = 0; j0 <= Ny; j0 += pgd::kTileY)
-        for (int i0 = 0; i0 <= Nx; i0 += pgd::kTileX) {
-          std::vector<int4> ent[2];
-          std::vector<int4> tsg;
-          bool any = false;
-          for (int r = 0; r < pgd::kTileY; ++r) {
-            int off = r * pgd::kTileRowStage;
-            int4 seg = make_int4(-1, 0, 0, 0);
-            int seg_next = -1;   // CSR slot that continues the open segment
-            for (int cc = 0; cc < pgd::kTileX; ++cc) {
-              const int i = i0 + cc, j = j0 + r;
-              const int cls = (i + j) % 2;
-              int4 e = make_int4(-1, 0, 0, 0);
-              if (i <= Nx && j <= Ny && st_of[j * sx + i].x >= 0) {
-                const int4 v = st_of[j * sx + i];
-                e = make_int4(v.x, v.y, v.z, off);
-                any = true;
-                if (seg.x >= 0 && v.z == seg_next) {
-                  seg.z += runlen[cls];
-                } else {
-                  if (seg.x >= 0) tsg.push_back(seg);
-                  seg = make_int4(off, v.z, runlen[cls], 0);
-                }
-                seg_next = v.z + runlen[cls];
-              } else if (seg.x >= 0) {
-                tsg.push_back(seg);
-                seg = make_int4(-1, 0, 0, 0);
-              }
-              ent[cls].push_back(e);
-              off += runlen[cls];
-            }
-            if (seg.x >= 0) tsg.push_back(seg);
-          }
-          if (!any) continue;
-          if (ent[0].size() != 64 || ent[1].size() != 64) return set_err(c, PG_ERR_STATE, "internal: tile classes");
-          tiles.push_back(make_int4(i0, j0, (int)segs.size(), (int)tsg.size()));
-          tnodes.insert(tnodes.end(), ent[0].begin(), ent[0].end());
-          tnodes.insert(tnodes.end(), ent[1].begin(), ent[1].end());
-          segs.insert(segs.end(), tsg.begin(), tsg.end());
-        }
-      PG_TRY(upload(c, tiles, &c->tiles));
-      PG_TRY(upload(c, tnodes, &c->tnodes));
-      PG_TRY(upload(c, segs, &c->tsegs));
-      c->n_tiles = (int)tiles.size();
-    }
-    // 3D tiles of 4 x 4 x 4 grid nodes (pg_tile.cuh): per tile {i0, j0, k0, 0} and {first
-    // segment, segments, 0, 0}; 64 node entries (x fastest) with their run's stage offset (a
-    // node's three rows are one run of 135 values); the contiguous CSR segments of each x-row
-    if (dim == 3 && grid_ok) {
-      std::vector<int4> st_of(s.n_std, make_int4(-1, 0, 0, 0));
-      for (const int4& v : by_class[0]) st_of[v.x] = v;
-      constexpr int T3 = pgd::kT3, RUN = pgd::kT3Run;
-      std::vector<int4> tiles, tnodes, segs;
-      for (int k0 = 0; k0 <= Nz; k0 += T3)
-        for (int j0 = 0; j0 <= Ny; j0 += T3)
-          for (int i0 = 0; i0 <= Nx; i0 += T3) {
-            std::vector<int4> ent, tsg;
-            bool any = false;
-            for (int lk = 0; lk < T3; ++lk)
-              for (int lj = 0; lj < T3; ++lj) {
-                int4 seg = make_int4(-1, 0, 0, 0);
-                int seg_next = -1;
-                for (int li = 0; li < T3; ++li) {
-                  const int i = i0 + li, j = j0 + lj, k = k0 + lk;
-                  const int off = ((lk * T3 + lj) * T3 + li) * RUN;
-                  int4 e = make_int4(-1, 0, 0, 0);
-                  if (i <= Nx && j <= Ny && k <= Nz && st_of[k * sxy + j * sx + i].x >= 0) {
-                    const int4 v = st_of[k * sxy + j * sx + i];
-                    e = make_int4(v.x, v.y, v.z, off);
-                    any = true;
-                    if (seg.x >= 0 && v.z == seg_next) seg.z += RUN;
-                    else {
-                      if (seg.x >= 0) tsg.push_back(seg);
-                      seg = make_int4(off, v.z, RUN, 0);
-                    }
-                    seg_next = v.z + RUN;
-                  } else if (seg.x >= 0) {
-                    tsg.push_back(seg);
-                    seg = make_int4(-1, 0, 0, 0);
-                  }
-                  ent.push_back(e);
-                }
-                if (seg.x >= 0) tsg.push_back(seg);
-              }
-            if (!any) continue;
-            tiles.push_back(make_int4(i0, j0, k0, 0));
-            tiles.push_back(make_int4((int)segs.size(), (int)tsg.size(), 0, 0));
-            tnodes.insert(tnodes.end(), ent.begin(), ent.end());
-            segs.insert(segs.end(), tsg.begin(), tsg.end());
-          }
-      PG_TRY(upload(c, tiles, &c->tiles));
-      PG_TRY(upload(c, tnodes, &c->tnodes));
-      PG_TRY(upload(c, segs, &c->tsegs));
-      c->n_tiles = (int)tiles.size() / 2;
-    }
-    std::vector<int> rest;
-    maxnb_general = 1;
-    for (int a = 0; a < s.n_dn; ++a)
-      if (!in_stencil[a]) { rest.push_back(a); maxnb_general = std::max(maxnb_general, s.dn_nbr_off[a + 1] - s.dn_nbr_off[a]); }
-    // general nodes grouped by shape (cut adjacent elements, then all adjacent elements, both
-    // descending; node order within a group) so the lane groups of a warp walk alike entries
-    auto n_cut_adj = [&](int a) {
-      int k = 0;
-      for (int j = s.dn_adj_off[a]; j < s.dn_adj_off[a + 1]; ++j) k += s.cut_of[s.dn_adj[j] >> 5] >= 0;
-      return k;
-    };
-    std::stable_sort(rest.begin(), rest.end(), [&](int x, int y) {
-      const int cx = n_cut_adj(x), cy = n_cut_adj(y);
-      if (cx != cy) return cx > cy;
-      return (s.dn_adj_off[x + 1] - s.dn_adj_off[x]) > (s.dn_adj_off[y + 1] - s.dn_adj_off[y]);
+    for (const int4& v : by_node) fast.push_back(s.node_dn[v.x]);
+    // general nodes: those on no cohesive element first, then by their number of neighbours, so
+    // that the lane groups of a warp walk alike rows
+    std::vector<char> on_coh(s.n_dn, 0);
+    for (int cc = 0; cc < s.ncut; ++cc)
+      for (int ce = s.cut_coh_off[cc]; ce < s.cut_coh_off[cc + 1]; ++ce)
+        for (int q = s.coh_local_off[ce]; q < s.coh_local_off[ce + 1]; ++q)
+          on_coh[s.node_dn[s.cut_nodes[s.cut_node_off[cc] + s.coh_local[q]]]] = 1;
+    for (int a = 0; a < s.n_dn; ++a) if (!in_stencil[a]) slow.push_back(a);
+    std::stable_sort(slow.begin(), slow.end(), [&](int x, int y) {
+      if (on_coh[x] != on_coh[y]) return on_coh[x] < on_coh[y];
+      return (s.dn_nbr_off[x + 1] - s.dn_nbr_off[x]) > (s.dn_nbr_off[y + 1] - s.dn_nbr_off[y]);
     });
-    slow.swap(rest);
-    fast.clear();
-    for (auto& v : stencil) if (v.x >= 0) fast.push_back(s.node_dn[v.x]);
-    c->grid = pgd::GridInfo{Nx, Ny, Nz};
+    c->P.n_gen_plain = 0;
+    for (int a : slow) c->P.n_gen_plain += !on_coh[a];
+    c->P.nx = Nx;
+    c->P.ny = Ny;
   }
   // cut-element scratch layout
   std::vector<long long> ke_off(s.ncut + 1, 0);
@@ -413,8 +370,9 @@ int pg_upload(pg_ctx* c) {
   c->cut_scratch = ke_off[s.ncut];
   c->n_coh_qp = (int)s.cqp_wgt.size();
 
-  // descriptors of the general rows (k_rows_general)
-  std::vector<int4> gdesc, adesc;
+  // descriptors of the general rows
+  std::vector<int4> gdesc, adesc, gnd;
+  int stat_slots = 0;
   std::vector<int> growd;
   std::vector<int4> aresd;   // per entry: uncut {element nodes}, cut {cut element, first node, cohesive place, 0}
   for (int a : slow) {
@@ -431,6 +389,18 @@ int pg_upload(pg_ctx* c) {
       rows[2][q] = rf ? s.rp[1][rr] : s.rp[3][rr];
     }
     for (int t = 0; t < 3; ++t) for (int q = 0; q < dim; ++q) growd.push_back(rows[t][q]);
+    {
+      // regular: every row and neighbour DOF free, so the rows are one run of K_ff
+      const int nn = gdesc.back().w, g0 = rows[0][0];
+      bool regular = true;
+      for (int k = gdesc.back().z; k < gdesc.back().z + nn; ++k) regular = regular && nbr_mask[k] == (1 << dim) - 1;
+      for (int q = 0; regular && q < dim; ++q)
+        regular = rows[0][q] == g0 + q && g0 + q < s.n_free && rows[1][q] == rows[1][0] + q * nn * dim &&
+                  s.rp[0][g0 + q + 1] - s.rp[0][g0 + q] == nn * dim;
+      gnd.push_back(make_int4(stat_slots, nn | (regular ? 1 << 16 : 0), regular ? rows[1][0] : 0, regular ? g0 : 0));
+      gnd.push_back(make_int4(0, 0, 0, 0));
+      stat_slots += nn;
+    }
     // cut elements first, then uncut ones, each in adjacency order
     for (int pass = 0; pass < 2; ++pass)
     for (int k = s.dn_adj_off[a]; k < s.dn_adj_off[a + 1]; ++k) {
@@ -452,11 +422,6 @@ int pg_upload(pg_ctx* c) {
         aresd.push_back(make_int4(cc, s.cut_node_off[cc], cpa, 0));
       }
     }
-    // k_rows_general walks a node's cut entries until the first uncut one: every node's entries
-    // must be cut-first
-    for (size_t k = (size_t)gdesc.back().x + 1; k < adesc.size(); ++k)
-      if ((adesc[k].y >> 8) != 0 && (adesc[k - 1].y >> 8) == 0)
-        return set_err(c, PG_ERR_STATE, "internal: a cut entry after an uncut one in a general row");
   }
 
   // ---- device residency
@@ -464,27 +429,24 @@ int pg_upload(pg_ctx* c) {
   P.dim = dim; P.npe = s.npe; P.nvoigt = s.nvoigt;
   P.n_nodes = n_nodes; P.ne = s.ne; P.ncut = s.ncut; P.n_dn = s.n_dn;
   P.n_free = s.n_free; P.n_const = s.n_const; P.subscale = s.desc.subscale;
-  for (int m = 0; m < 3; ++m) for (int i = 0; i < 36; ++i) { P.D[m][i] = s.D[m][i]; P.Df[m][i] = (float)s.D[m][i]; }
   P.coh.law = s.coh.law; P.coh.nvar = s.coh.nvar; P.coh.sigma_c = s.coh.sigma_c; P.coh.delta_c1 = s.coh.delta_c1;
   P.coh.delta_c2 = s.coh.delta_c2; P.coh.delta_cn = s.coh.delta_cn; P.coh.delta_ct = s.coh.delta_ct; P.coh.q = s.coh.q;
   P.coh.delta_c = s.coh.delta_c; P.coh.beta2 = s.coh.beta2; P.coh.alpha = s.coh.alpha; P.coh.delta_c3 = s.coh.delta_c3;
   {
     std::vector<double> Dh(108);
-    std::vector<float> Dfh(108);
-    for (int m = 0; m < 3; ++m) for (int i = 0; i < 36; ++i) { Dh[m * 36 + i] = s.D[m][i]; Dfh[m * 36 + i] = (float)s.D[m][i]; }
+    for (int m = 0; m < 3; ++m) for (int i = 0; i < 36; ++i) Dh[m * 36 + i] = s.D[m][i];
     PG_TRY(upload(c, Dh, &P.Dd));
-    PG_TRY(upload(c, Dfh, &P.Dfd));
   }
-  if ((dim == 2 ? pgl::tile_consts<2>(c, P) : pgl::tile_consts<3>(c, P)) != 0)
-    return set_err(c, PG_ERR_DEVICE, "tile shape constants failed");
-  std::vector<float> Xf(s.X.begin(), s.X.end());
+  if (!stencil.empty()) PG_TRY(structured_constants(c));
+  P.n_snode = (int)stencil.size();
+  P.n_chunk = (int)chunks.size();
+  PG_TRY(upload(c, stencil, &P.snode));
+  PG_TRY(upload(c, chunks, &P.chunk));
   PG_TRY(upload(c, s.X, &P.X));
-  PG_TRY(upload(c, Xf, &P.Xf));
   PG_TRY(upload(c, s.conn, &P.conn));
   PG_TRY(upload(c, s.elem_mat, &P.emat));
   PG_TRY(upload(c, s.cut_of, &P.cut_of));
   PG_TRY(upload(c, s.node_dof, &P.node_dof));
-  PG_TRY(upload(c, s.node_dn, &P.node_dn));
   PG_TRY(upload(c, s.cut_node_off, &P.cut_node_off));
   PG_TRY(upload(c, s.cut_nodes, &P.cut_nodes));
   // Device quadrature tables: the quadrature points of an affine (tri3 / tet4) sub-element of an
@@ -583,22 +545,10 @@ int pg_upload(pg_ctx* c) {
   PG_TRY(upload(c, nbr_mask, &P.dn_nbr_mask));
   PG_TRY(upload(c, s.dn_adj_off, &P.dn_adj_off));
   PG_TRY(upload(c, s.dn_adj, &P.dn_adj));
-  PG_TRY(upload(c, slot32, &P.adj_slot32));
-  PG_TRY(upload(c, slot_off, &P.adj_slot_off));
   PG_TRY(upload(c, slots, &P.adj_slots));
-  PG_TRY(upload(c, fast, &P.fast_dn));
-  PG_TRY(upload(c, slow, &P.slow_dn));
-  {
-    const int4* dst = nullptr;
-    PG_TRY(upload(c, stencil, &dst));
-    c->stencil = dst;
-    c->n_stencil = (int)stencil.size();
-  }
   c->fast_dn = fast;
   c->slow_dn = slow;
-
-  P.n_fast_dn = (int)fast.size(); P.n_slow_dn = (int)slow.size();
-  P.maxnb_general = maxnb_general;
+  P.n_slow_dn = (int)slow.size();
   PG_TRY(upload(c, gdesc, &P.gdesc));
   PG_TRY(upload(c, growd, &P.growd));
   PG_TRY(upload(c, adesc, &P.adesc));
@@ -623,7 +573,6 @@ int pg_upload(pg_ctx* c) {
           slot = ce * 32 + k;
         }
       }
-    PG_TRY(upload(c, ce_cut, &P.ce_cut));
     {
       // node ids of the cohesive elements' local nodes, laid out like coh_local
       std::vector<int> gnode(s.coh_local.size());
@@ -633,7 +582,6 @@ int pg_upload(pg_ctx* c) {
       PG_TRY(upload(c, gnode, &P.coh_gnode));
     }
     PG_TRY(upload(c, kc_off, &P.kc_off));
-    PG_TRY(upload(c, cohpos, &P.cohpos));
     kc_off_h = kc_off;
     cohpos_h = cohpos;
     double* dk;
@@ -641,9 +589,6 @@ int pg_upload(pg_ctx* c) {
     P.kcoh = dk;
     P.n_coh_el = n_ce;
     P.n_coh_qp = c->n_coh_qp;
-    int max_mn = 1;
-    for (int cc = 0; cc < s.ncut; ++cc) max_mn = std::max(max_mn, s.cut_node_off[cc + 1] - s.cut_node_off[cc]);
-    P.max_mn = max_mn;
   }
   // row positions: free DOFs of the earlier neighbours of every neighbour slot
   {
@@ -654,16 +599,7 @@ int pg_upload(pg_ctx* c) {
     }
     PG_TRY(upload(c, pre, &P.nbr_pre));
   }
-  // side: the structured tiles at the lowest priority; side2: the general chain at the highest
-  {
-    int least = 0, greatest = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, least) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, greatest) != cudaSuccess)
-      return set_err(c, PG_ERR_DEVICE, "stream creation failed");
-  }
   for (int b = 0; b < 4; ++b) {
-    PG_TRY(upload(c, s.rp[b], &P.rp[b]));
     // (two more than there are: the solver's copies of value ranges end on 16-byte boundaries)
     PG_TRY(dalloc(c, s.ci[b].size() + 2, &P.val[b]));
   }
@@ -697,105 +633,79 @@ int pg_upload(pg_ctx* c) {
   PG_TRY(dalloc(c, 1, &c->d_err));
   P.err = c->d_err;
   PG_TRY(dalloc(c, 1024, &c->d_red));
-  // Static part of the general rows.  tri3 / tet4: every general node gets one, holding its cut
-  // and uncut elements' volumetric blocks (every bulk law is linear elastic, so these do not
-  // depend on the state; k_general_static forms them once), and an assembly adds only the
-  // cohesive blocks.  quad4: only the general nodes with cut adjacent elements, sorted first, so
-  // they form the prefix [0, n_stat).  Each gets its neighbour slots' blocks (slab layout), the
-  // slot node ids and a macroscale-strain response.
+  // Static image of the general rows (k_general_static), the node ids of its slots, the cohesive
+  // contributions of every slot in adjacency order and the nodes' traction lists
   {
-    const int nv = (dim == 2) ? 3 : 6;
-    const bool full_static = s.etype != pg::QUAD4;
-    int n_stat = 0;
+    const int nv = (dim == 2) ? 3 : 6, D2 = dim * dim;
+    std::vector<int> stat_node, gblk_cl(1, 0), gcl, tl;
+    stat_node.reserve(stat_slots);
+    gblk_cl.reserve(stat_slots + 1);
+    std::vector<std::vector<int>> bcl;
     for (size_t i = 0; i < slow.size(); ++i) {
       const int4 gd = gdesc[i];
-      const bool has_cut = gd.y > 0 && (adesc[gd.x].y >> 8) != 0;   // entries are cut-first
-      if (has_cut && (int)i != n_stat) return set_err(c, PG_ERR_STATE, "internal: general nodes next to cut elements are not a prefix");
-      if (has_cut) ++n_stat;
-    }
-    if (full_static) n_stat = (int)slow.size();
-    std::vector<int> stat_off(n_stat + 1, 0), stat_node;
-    for (int i = 0; i < n_stat; ++i) {
-      const int4 gd = gdesc[i];
-      stat_off[i + 1] = stat_off[i] + gd.w;
       for (int k = gd.z; k < gd.z + gd.w; ++k) stat_node.push_back(s.dn_node[s.dn_nbr[k]]);
+      if ((int)i < P.n_gen_plain) {
+        gblk_cl.insert(gblk_cl.end(), gd.w, 0);
+        continue;
+      }
+      bcl.assign(gd.w, std::vector<int>());
+      gnd[2 * i + 1].x = (int)tl.size();
+      for (int k = gd.x; k < gd.x + gd.y; ++k) {
+        const int4 ad = adesc[k], ax = aresd[k];
+        const int mn = ad.y >> 8;
+        if (mn == 0) continue;   // uncut: in the static image
+        const int cpa = ax.z;
+        if (cpa < 0) continue;
+        const int ce = cpa >> 5, n1 = cpa & 31, nh = s.coh_nh[ce];
+        for (int b = 0; b < mn; ++b) {
+          const int cpb = cohpos_h[ax.y + b];
+          if (cpb < 0 || (cpb >> 5) != ce) continue;
+          const int n2 = cpb & 31;
+          const int off = kc_off_h[ce] + ((n1 % nh) * nh + (n2 % nh)) * D2;
+          const int neg = ((n1 >= nh) == (n2 >= nh)) ? 0 : 1;
+          bcl[slots[ad.z + b]].push_back(off * 2 + neg);
+        }
+        const int toff = kc_off_h[ce] + nh * nh * D2 + (n1 % nh) * dim;
+        tl.push_back(toff * 2 + ((n1 >= nh) ? 0 : 1));
+      }
+      for (int k = 0; k < gd.w; ++k) {
+        gcl.insert(gcl.end(), bcl[k].begin(), bcl[k].end());
+        gblk_cl.push_back((int)gcl.size());
+      }
+      gnd[2 * i + 1].y = (int)tl.size() - gnd[2 * i + 1].x;
     }
-    P.n_stat = n_stat;
-    PG_TRY(upload(c, stat_off, &P.stat_slot_off));
+    for (size_t k = 0; k < aresd.size() && P.n_gen_plain > 0; ++k)
+      if ((int)k < gdesc[P.n_gen_plain - 1].x + gdesc[P.n_gen_plain - 1].y && (adesc[k].y >> 8) != 0 && aresd[k].z >= 0)
+        return set_err(c, PG_ERR_STATE, "internal: a node on a cohesive element among the plain general nodes");
+    PG_TRY(upload(c, gnd, &P.gnd));
     PG_TRY(upload(c, stat_node, &P.stat_node));
+    PG_TRY(upload(c, gblk_cl, &P.gblk_cl));
+    PG_TRY(upload(c, gcl, &P.gcl));
+    PG_TRY(upload(c, tl, &P.gnode_tl));
     double* dst = nullptr;
     double* dsg = nullptr;
-    PG_TRY(dalloc(c, (size_t)stat_off[n_stat] * dim * dim, &dst));
-    PG_TRY(dalloc(c, (size_t)n_stat * dim * nv, &dsg));
+    PG_TRY(dalloc(c, (size_t)stat_slots * D2, &dst));
+    PG_TRY(dalloc(c, slow.size() * dim * nv, &dsg));
     P.stat = dst;
     P.stat_g = dsg;
-    // Block-parallel general rows (pg_general.cuh; tri3 / tet4): one block per (general node,
-    // neighbour slot) with its static index and its cohesive contributions in adjacency order,
-    // and per node the traction list (the uncut elements are in the static image)
-    if (s.etype != pg::QUAD4) {
-      const int D2 = dim * dim;
-      std::vector<int4> gblk;
-      std::vector<int> gblk_cl(1, 0), gcl, tl_off(1, 0), tl;
-      std::vector<std::vector<int>> bcl;
-      for (size_t i = 0; i < slow.size(); ++i) {
-        const int4 gd = gdesc[i];
-        bcl.assign(gd.w, std::vector<int>());
-        for (int k = gd.x; k < gd.x + gd.y; ++k) {
-          const int4 ad = adesc[k], ax = aresd[k];
-          const int mn = ad.y >> 8;
-          if (mn == 0) continue;   // uncut: in the static image
-          const int cpa = ax.z;
-          if (cpa < 0) continue;
-          const int ce = cpa >> 5, n1 = cpa & 31, nh = s.coh_nh[ce];
-          for (int b = 0; b < mn; ++b) {
-            const int cpb = cohpos_h[ax.y + b];
-            if (cpb < 0 || (cpb >> 5) != ce) continue;
-            const int n2 = cpb & 31;
-            const int off = kc_off_h[ce] + ((n1 % nh) * nh + (n2 % nh)) * D2;
-            const int neg = ((n1 >= nh) == (n2 >= nh)) ? 0 : 1;
-            bcl[slots[ad.z + b]].push_back(off * 2 + neg);
-          }
-          const int toff = kc_off_h[ce] + nh * nh * D2 + (n1 % nh) * dim;
-          tl.push_back(toff * 2 + ((n1 >= nh) ? 0 : 1));
-        }
-        for (int k = 0; k < gd.w; ++k) {
-          gblk.push_back(make_int4((int)i, k, stat_off[i] + k, 0));
-          gcl.insert(gcl.end(), bcl[k].begin(), bcl[k].end());
-          gblk_cl.push_back((int)gcl.size());
-        }
-        tl_off.push_back((int)tl.size());
-      }
-      P.n_gblk = (int)gblk.size();
-      PG_TRY(upload(c, gblk, &P.gblk));
-      PG_TRY(upload(c, gblk_cl, &P.gblk_cl));
-      PG_TRY(upload(c, gcl, &P.gcl));
-      PG_TRY(upload(c, tl_off, &P.gnode_tl_off));
-      PG_TRY(upload(c, tl, &P.gnode_tl));
-    }
-    c->stat_doubles = (long long)stat_off[n_stat] * dim * dim + (long long)n_stat * dim * nv;
+    double* dg = nullptr;
     if (s.ncut > 0) {
-      double* dg = nullptr;
       PG_TRY(dalloc(c, (size_t)re_off[s.ncut] / dim * dim * nv, &dg));
       P.gmac = dg;
-      if (dim == 2) { pgl::cut_volumetric<2>(c, P, dg); pgl::general_static<2>(c, P, dst, dsg); }
-      else { pgl::cut_volumetric<3>(c, P, dg); pgl::general_static<3>(c, P, dst, dsg); }
-      int herr = 0;
-      cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->up);
-      if (cudaStreamSynchronize(c->up) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "cut-element set-up kernel failed");
-      if (herr) return set_err(c, PG_ERR_NONFINITE, "non-finite cut-element stiffness at set-up");
-      // the per-element blocks are reduced: give their memory back
-      for (double* p : {dke, dg}) pg_untrack_free(c, p);
-      P.ke = nullptr;
-      P.gmac = nullptr;
-    } else if (full_static && n_stat > 0) {
-      // no cut elements: the image holds the uncut elements alone
-      if (dim == 2) pgl::general_static<2>(c, P, dst, dsg);
-      else pgl::general_static<3>(c, P, dst, dsg);
-      int herr = 0;
-      cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->up);
-      if (cudaStreamSynchronize(c->up) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "general-row set-up kernel failed");
-      if (herr) return set_err(c, PG_ERR_NONFINITE, "non-finite general-row stiffness at set-up");
+      if (dim == 2) pgl::cut_volumetric<2>(c, P, dg);
+      else pgl::cut_volumetric<3>(c, P, dg);
     }
+    if (dim == 2) pgl::general_static<2>(c, P, dst, dsg);
+    else pgl::general_static<3>(c, P, dst, dsg);
+    int herr = 0;
+    cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->up);
+    if (cudaStreamSynchronize(c->up) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "general-row set-up kernel failed");
+    if (herr) return set_err(c, PG_ERR_NONFINITE, "non-finite stiffness at set-up");
+    // the per-element blocks are reduced: give their memory back
+    pg_untrack_free(c, dke);
+    if (dg) pg_untrack_free(c, dg);
+    P.ke = nullptr;
+    P.gmac = nullptr;
   }
   return pg_alloc_sync(c);
 }
@@ -843,15 +753,10 @@ int pg_set_timing(pg_ctx* c, int on) {
 int pg_kernel_times(pg_ctx* c, float* ms) {
   if (!c || !ms || !c->ev[0]) return set_err(c, PG_ERR_STATE, "nothing was launched");
   if (!c->timed_last) return set_err(c, PG_ERR_STATE, "the last assembly ran with timing off (pg_set_timing)");
-  if (cudaEventSynchronize(c->ev[5]) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "event wait failed");
-  // [0] cohesive elements and element records, [1] stencil rows (2D: from the start, on their
-  // own stream, concurrent with [0] and [2]; 3D: after [0]), [2] general rows (after [0] in 2D,
-  // after [1] in 3D), [3] whole assembly
-  const bool seq = c->s.dim == 3;
-  cudaEventElapsedTime(&ms[0], c->ev[0], c->ev[3]);
-  cudaEventElapsedTime(&ms[1], seq ? c->ev[3] : c->ev[0], c->ev[1]);
-  cudaEventElapsedTime(&ms[2], seq ? c->ev[1] : c->ev[3], c->ev[4]);
-  cudaEventElapsedTime(&ms[3], c->ev[0], c->ev[5]);
+  if (cudaEventSynchronize(c->ev[4]) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "event wait failed");
+  // [0] cohesive elements, [1] structured rows, [2] general rows, [3] whole assembly
+  for (int k = 0; k < 3; ++k) cudaEventElapsedTime(&ms[k], c->ev[k], c->ev[k + 1]);
+  cudaEventElapsedTime(&ms[3], c->ev[0], c->ev[4]);
   return 0;
 }
 
@@ -859,18 +764,13 @@ void pg_destroy(pg_ctx* c) {
   if (!c) return;
   // work of this context still in flight finishes before its memory goes back to the pool
   cudaStreamSynchronize(c->stream);
-  if (c->side) cudaStreamSynchronize(c->side);
-  if (c->side2) cudaStreamSynchronize(c->side2);
   if (c->pcg.stream) cudaStreamSynchronize(c->pcg.stream);
   if (c->pcg.stream) cudaStreamDestroy(c->pcg.stream);
   for (cudaEvent_t e : {c->pcg.ev, c->pcg.evc[0], c->pcg.evc[1]}) if (e) cudaEventDestroy(e);
   if (c->pcg.hflag) cudaFreeHost(c->pcg.hflag);
-  for (int i = 0; i < 6; ++i) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
-  if (c->side) cudaStreamDestroy(c->side);
-  if (c->side2) cudaStreamDestroy(c->side2);
+  for (cudaEvent_t e : c->ev) if (e) cudaEventDestroy(e);
   for (void* p : c->allocs) cudaFreeAsync(p, c->up);
   if (c->up) cudaStreamDestroy(c->up);   // released once the frees have run
-  delete c->t3c;
   delete c;
 }
 

@@ -5,14 +5,12 @@
 // committed and trial internal variables, the cut-element scratch and the solver workspace.
 #pragma once
 
-#include "pg_stencil.cuh"
+#include "pg_device.cuh"
 #include "pg_setup.h"
 #include "../../include/pigfem_b200.h"
 
 #include <string>
 #include <vector>
-
-namespace pgd { struct Tile3Const; }
 
 // Workspace of the Jacobi-preconditioned CG on K_ff (pg_solver.cu), allocated on first use.
 struct PcgWork {
@@ -47,13 +45,9 @@ struct pg_ctx {
   int* d_err = nullptr;
   double* d_red = nullptr;  // residual-norm partials
   long long cut_scratch = 0;   // doubles of the cut elements' set-up blocks (released after set-up)
-  long long stat_doubles = 0;  // doubles of the general rows' static part
   int max_nd = 0;
-  int maxnb_fast = 0;
   int n_coh_qp = 0;
   bool assembled = false;
-  pgd::Tile3Const* t3c = nullptr;         // 3D tiles' shape constants: host copy (kernel parameter)
-  const pgd::Tile3Const* d_t3c = nullptr; // and device copy (batches)
   bool timed_last = false;   // the last assembly recorded every timing event (pg_kernel_times)
   double prep_ms = -1.0;   // device time of the preprocessing passes (pg_create_prep_device), -1 if none ran
   // PG_KEEP_STATIC: the first CSR value of each block from which a later assembly can change
@@ -63,25 +57,12 @@ struct pg_ctx {
   double* kept[4] = {nullptr, nullptr, nullptr, nullptr};
   bool kept_fp32 = false, kept_valid = false;
   std::vector<int> fast_dn, slow_dn;
-  int tile_nodes = 128;
   int max_cut_qp = 1, max_cut_nodes = 1;
   const int* cut_list[2] = {nullptr, nullptr};
   int n_cut_list[2] = {0, 0};
   int cut_cls_qp[2] = {1, 1}, cut_cls_nodes[2] = {1, 1};
-  const int4* stencil = nullptr;
-  int n_stencil = 0;
-  // 2D tiles of the stencil rows (pg_tile.cuh): per tile {i0, j0, first segment, segments}, per
-  // tile 128 node entries {node, first DOF, first CSR slot, stage offset}, the store segments
-  const int4* tiles = nullptr;
-  const int4* tnodes = nullptr;
-  const int4* tsegs = nullptr;
-  int n_tiles = 0;
-  pgd::GridInfo grid{0, 0, 0};
   bool timing = false;
-  cudaStream_t side = nullptr;    // 2D: the structured tiles (lowest stream priority)
-  cudaStream_t side2 = nullptr;   // 2D: cohesive elements, records and general rows (highest priority)
-  // fork, tiles done, (unused), first kernel done, general rows done, join
-  cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // start, cohesive, structured, general done, end
   PcgWork pcg;
   // material sensitivity pass (pg_sens.cu): made on its first call
   struct SensWork {

@@ -36,28 +36,24 @@ struct DevProblem {
   int n_nodes, ne, ncut, n_dn;
   int n_free, n_const;
   int subscale;
-  double D[3][36];    // bulk materials: 0 matrix, 1 fiber, 2 bounding plies
-  float Df[3][36];
-  const double* Dd;   // D of the three bulk materials in device memory (3 x 36), read through the L1
-  const float* Dfd;
-  // 2D structured tiles (pg_tile.cuh): every uncut element of the uniform grid is one of four
-  // shapes (2 x cell parity + element in the cell); per shape the gradients of its three nodes, its
-  // weight J W, and its element matrix per bulk material ([(la * 2 + q) * 6 + lb * 2 + q2], FP64
-  // and the FP32-mixed products), formed once at upload by the element code itself
-  double tile_g[4][3][2];
-  double tile_w[4];
-  double tile_ke[4][3][36];
-  float tile_kef[4][3][36];
+  const double* Dd;   // D of the bulk materials (3 x 36): 0 matrix, 1 fiber, 2 bounding plies
+  // structured rows (pg_rows.cuh): the pattern of their CSR values ([precision][material][shift]
+  // [period]), their coefficients in the residual ([material][class][row][slot][component]) and
+  // macroscale response ([material][class][row][strain]); the CSR chunks and the nodes
+  const double* pat;
+  const double* srow;
+  const double* sg;
+  const int4* chunk; int n_chunk;
+  const int4* snode; int n_snode;
+  int nx, ny;         // cells per direction
   CohConst coh;
   // geometry / state
   const double* X;    // n_nodes * dim
-  const float* Xf;    // n_nodes * dim (FP32 copy for the mixed path)
   const double* U;    // n_nodes * dim, node-major (the reference's NodalData layout)
   const int* conn;    // ne * npe
   const int* emat;    // ne
   const int* cut_of;  // ne
   const int* node_dof;  // n_nodes * dim
-  const int* node_dn;   // n_nodes
   // cut elements
   const int* cut_node_off; const int* cut_nodes;
   const int* cut_qp_off; const double* qp_wgt; const int* qp_mat; const int* qp_grad_off; const double* qp_grad;
@@ -68,13 +64,13 @@ struct DevProblem {
   const int* re_off;        // per cut element: offset of its first node's rows (nodes x dim)
   double* ke;               // set-up only: volumetric element matrices of the cut elements
   const double* gmac;       // set-up only: macroscale-strain response of the cut elements
-  // Static part of the general rows next to cut elements (the first n_stat general nodes): the
-  // cut elements' volumetric blocks summed per neighbour slot, in the slab layout [slot][q][d]
-  // (stat, from stat_slot_off[node] slots on), the node id of each slot (stat_node) and the
-  // summed macroscale-strain response (stat_g, dim x nvoigt per node).  The bulk laws are linear
-  // elastic, so these do not depend on the state; k_general_static forms them once at set-up.
-  int n_stat;
-  const int* stat_slot_off;
+  // general rows (pg_rows.cuh): per node two int4 (gnd: gen_node's descriptor), its rows' static
+  // image (stat, laid out like the CSR rows), the node id of each slot (stat_node) and the
+  // macroscale-strain response (stat_g, dim x nvoigt); the first n_gen_plain nodes are on no
+  // cohesive element.  The bulk laws are linear elastic, so these do not depend on the state;
+  // k_general_static forms them once at set-up.
+  const int4* gnd;
+  int n_gen_plain;
   const int* stat_node;
   const double* stat;
   const double* stat_g;
@@ -84,33 +80,28 @@ struct DevProblem {
   // row ownership
   const int* dn_node; const int* dn_nbr_off; const uint8_t* dn_nbr_mask;  // free-DOF bits of each neighbour
   const int* dn_adj_off; const int* dn_adj;      // adjacent (element << 5 | local node)
-  const int* adj_slot32;                         // uncut elements: neighbour slot of each element node, 8 bits each
-  const int* adj_slot_off; const uint8_t* adj_slots;  // all elements: neighbour slot of each element node
-  const int* fast_dn; int n_fast_dn;             // DOF nodes whose elements are all uncut
-  const int* tile_elem_off; const int* tile_elems; int tile_max_elems;  // elements each tile of fast nodes touches
-  const uint16_t* adj_local;                     // tile-local index of each adjacency entry's element
-  const int* slow_dn; int n_slow_dn;             // the remaining DOF nodes
-  // Block-parallel general rows (pg_general.cuh; tri3 / tet4 meshes): one block per (general
-  // node, neighbour slot), node-major: {node, slot, static index, -}; its cohesive contributions
-  // [gblk_cl[b], gblk_cl[b + 1]) as (kcoh offset << 1 | negative) in adjacency order; per general
-  // node the residual's traction list (kcoh offset << 1 | negative), in adjacency order.
-  int n_gblk;
-  const int4* gblk; const int* gblk_cl; const int* gcl;
-  const int* gnode_tl_off; const int* gnode_tl;
-  int maxnb_general;                             // slab slots per node in k_rows_general
-  const int4* gdesc; const int* growd; const int4* adesc; const int4* aresd;  // k_rows_general descriptors
+  const uint8_t* adj_slots;                      // cut elements' entries: neighbour slot of each element node
+  int n_slow_dn;                                 // the general DOF nodes
+  // cohesive contributions of the general rows: per static slot b the blocks
+  // [gblk_cl[b], gblk_cl[b + 1]) of gcl, as (kcoh offset << 1 | negative) in adjacency order; the
+  // nodes' tractions likewise in gnode_tl
+  const int* gblk_cl; const int* gcl;
+  const int* gnode_tl;
+  // descriptors of the general nodes and their adjacent elements:
+  //   gdesc[node]   {adjacency begin, adjacency count, neighbour begin, neighbour count}
+  //   growd[node]   3*dim ints: global DOF of each row, first slot in the row's F block, in its C block
+  //   adesc[entry]  {element, local node | nodes of a cut element << 8, slots (uncut: 8 bits per node;
+  //                 cut: offset into adj_slots), material (uncut)}
+  //   aresd[entry]  uncut {element nodes (-1 padded)}; cut {cut element, its first node in cut_nodes, -, 0}
+  const int4* gdesc; const int* growd; const int4* adesc; const int4* aresd;
   // cohesive points
   int n_coh_qp;
   int n_coh_el;                                  // cohesive elements
-  const int* ce_cut;                             // cut element of each cohesive element
   const int* coh_gnode;                          // node id of every cohesive element's local node ('-' then '+', at coh_local_off)
   const int* kc_off;                             // per cohesive element: offset of its blocks in kcoh
   double* kcoh;                                  // per call: cohesive blocks B_ab and tractions t_a
-  const int* cohpos;                             // per cut-element local node: (cohesive element << 5 | position) or -1
   const int* nbr_pre;                            // per neighbour slot: free DOFs of the earlier neighbours
-  int max_mn;                                    // most nodes of a cut element
   // outputs: CSR values of the four blocks and the two residual parts
-  const int* rp[4];
   double* val[4];
   double* Pf; double* Pp;
   // per-call

@@ -1,18 +1,13 @@
-// pg_kernels.cuh -- the assembly kernels.
+// pg_kernels.cuh -- element-level kernels and their set-up (the rows are in pg_rows.cuh).
 //
-//   k_coh_elements   one lane per cohesive quadrature point, the lanes of an element together:
+//   coh_element      one lane per cohesive quadrature point, the lanes of an element together:
 //                    opening delta = R sum_n N_n (U+ - U-), the traction-separation law with its
 //                    internal-variable update and damage zone, and the element's cohesive blocks
 //                    and tractions (src/Utilities.cpp:528-594).  FP64.
 //   k_cut_volumetric run once at set-up: the cut elements' volumetric (linear, state-independent)
 //                    element matrices from sub-element quadrature with enriched B-matrices
 //                    (src/Assembler.cpp:223-274), cached for every later assembly.  FP64.
-//   k_rows_general   one lane group per DOF node (row owner) for every node the structured stencil
-//                    path (pg_stencil.cuh) does not take: boundary rows, nodes of cut elements and
-//                    enrichment nodes; uncut elements are recomputed from node coordinates; for cut
-//                    elements the cached volumetric block row is combined with the nodal
-//                    displacements and the cohesive elements' blocks (src/Assembler.cpp:278-365).
-//                    Every CSR value is written once.
+//   k_general_static run once at set-up: the static image of the rows pg_rows.cuh calls general.
 // No atomics anywhere: every row has one owner and sums in a fixed order, so results are
 // bit-reproducible from run to run.
 #pragma once
@@ -20,6 +15,8 @@
 #include "pg_device.cuh"
 
 namespace pgd {
+
+template <int N> struct IntC { static constexpr int value = N; };
 
 // Geometry of an affine simplex (tri3 / tet4): physical gradients g[n][d] and the Jacobian
 // determinant.  Jac(a,i) = sum_n dN_n/dr_a x_n[i] (Elem::transform_gradients), i.e. x_{a+1} - x_0;
@@ -129,90 +126,6 @@ __device__ __forceinline__ void add_strain(const T* g, const T* u, T* e) {
 __device__ __host__ inline double tri4_wsum() { return ((-0.28125 + 0.260416666666666666666666666666665) + 0.260416666666666666666666666666665) + 0.260416666666666666666666666666665; }
 __device__ __host__ inline double tet5_wsum() { return (((-0.8 + 0.45) + 0.45) + 0.45) + 0.45; }
 
-// Block (la, lb) of an uncut simplex with the given nodes: kb = w (B_la^T D B_lb) (WANT_K); with
-// want_r also the residual of row la, rv = w (B_la^T sigma).  Geometry from the node coordinates,
-// stress from U (+ eps_macro).
-template <int DIM, bool WANT_K = true>
-__device__ __forceinline__ void simplex_block(const DevProblem& P, int4 nodes, int la, int lb, const double* D,
-                                              double (*kb)[DIM], double* rv, bool want_r) {
-  constexpr int NPE = DIM + 1;
-  constexpr int NV = (DIM == 2) ? 3 : 6;
-  const int nd[4] = {nodes.x, nodes.y, nodes.z, nodes.w};
-  double x[NPE][DIM], g[NPE][DIM], J;
-#pragma unroll
-  for (int n = 0; n < NPE; ++n) load_node<DIM>(P.X, nd[n], x[n]);
-  simplex_geom<DIM, double>(x, g, &J);
-  const double wgt = J * ((DIM == 2) ? tri4_wsum() : tet5_wsum());
-  double ga[DIM], gb[DIM];
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) { ga[d] = g[0][d]; gb[d] = g[0][d]; }
-#pragma unroll
-  for (int n = 1; n < NPE; ++n) {
-    if (la == n)
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) ga[d] = g[n][d];
-    if (lb == n)
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) gb[d] = g[n][d];
-  }
-  if constexpr (WANT_K) {
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) {
-      double part[NV];
-      bt_d_row<DIM, double>(D, ga, q, part);
-#pragma unroll
-      for (int q2 = 0; q2 < DIM; ++q2) kb[q][q2] = wgt * part_b<DIM, double>(part, gb, q2);
-    }
-  }
-  if (want_r) {
-    double eps[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) eps[v] = 0.0;
-#pragma unroll
-    for (int n = 0; n < NPE; ++n) {
-      double u[DIM];
-      load_node<DIM>(P.U, nd[n], u);
-      add_strain<DIM, double>(g[n], u, eps);
-    }
-    if (P.subscale) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) eps[v] += P.eps_macro[v];
-    }
-    double sig[NV];
-    lei_stress<DIM, double>(D, eps, sig);
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) rv[q] = wgt * bt_sig<DIM, double>(ga, sig, q);
-  }
-}
-
-// Shared memory of one lane group of general_rows: slab_slots blocks of DIM x DIM, the node's
-// residual (4 doubles reserved), the per-slot residual partials of the static part
-// (slab_slots x DIM), then one scratch record per lane (general_lane_doubles).
-__host__ __device__ constexpr int general_lane_doubles(int dim, int npe) { return npe * dim * dim + dim + 2; }
-__host__ __device__ inline int general_scratch_offset(int slab_slots, int dim) {
-  return (slab_slots * dim * dim + 4 + slab_slots * dim + 1) & ~1;   // even: 16-byte aligned
-}
-__host__ __device__ inline int general_slab_doubles(int slab_slots, int dim, int lanes, int npe = 0) {
-  // even (16-byte aligned groups) and 2 mod 4, so consecutive groups start on different banks
-  if (npe == 0) npe = dim + 1;
-  int n = (general_scratch_offset(slab_slots, dim) + lanes * general_lane_doubles(dim, npe) + 1) & ~1;
-  return (n % 4 == 0) ? n + 2 : n;
-}
-
-// slab block += v (DIM x DIM); 16-byte shared-memory accesses in 2D
-template <int DIM>
-__device__ __forceinline__ void slab_add(double* ak, const double* v) {
-  if constexpr (DIM == 2) {
-    double2* a2 = reinterpret_cast<double2*>(ak);
-    double2 t0 = a2[0], t1 = a2[1];
-    t0.x += v[0]; t0.y += v[1]; t1.x += v[2]; t1.y += v[3];
-    a2[0] = t0; a2[1] = t1;
-  } else {
-#pragma unroll
-    for (int i = 0; i < DIM * DIM; ++i) ak[i] += v[i];
-  }
-}
-
 // Point qp of the quad4 2 x 2 Gauss rule (src/quad4.cpp:108-127: the edge points -+1/sqrt(3),
 // qp -> (qp % 2, qp / 2), weights 1 x 1) on the bilinear map of the nodes x: the physical
 // gradients g of the four shape functions (Jacobian J(a, i) = sum_k dN_k/dr_a x_k[i], its
@@ -239,406 +152,62 @@ __device__ __forceinline__ void quad4_point(const double (*x)[2], int qp, double
   *w = det * (1.0 * 1.0);
 }
 
-// Block row la of an uncut element with the given nodes: blk[b] = sum over its points of
-// w (B_la^T D B_b) for every element node b (NPE blocks of DIM x DIM, row-major), and its
-// residual rv = sum w (B_la^T sigma).  Simplices (NPE = DIM + 1) have constant gradients, so
-// their order-3 points are summed into one weight (the products of simplex_block); quad4
-// (DIM = 2, NPE = 4) sums its four Gauss points.  Geometry from the node coordinates, stress
-// from U (+ eps_macro).
-template <int DIM, int NPE = DIM + 1>
-__device__ __forceinline__ void uncut_block_row(const DevProblem& P, int4 nodes, int la, const double* D, double* blk,
-                                                double* rv) {
+// Rows of node la of an uncut element with corner coordinates x, added to blk (row q at blk + q *
+// pitch, node b's columns at b * DIM): sum over its points of w (B_la^T D B_b); and its
+// macroscale-strain response w (B_la^T D) added to G (DIM x NV).  Simplices have constant gradients,
+// so their order-3 points are summed into one weight; quad4 sums its four Gauss points first.
+template <int DIM, int NPE>
+__device__ __forceinline__ void element_rows(const double (*x)[DIM], int la, const double* D, double* blk, int pitch, double* G) {
   constexpr int NV = (DIM == 2) ? 3 : 6;
-  constexpr int D2 = DIM * DIM;
-  const int nd[4] = {nodes.x, nodes.y, nodes.z, nodes.w};
   if constexpr (DIM == 2 && NPE == 4) {
-    double x[4][2], u[4][2];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) { load_node<2>(P.X, nd[n], x[n]); load_node<2>(P.U, nd[n], u[n]); }
-    double kb[4][4], r[2] = {0.0, 0.0};
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) kb[b][i] = 0.0;
-#pragma unroll
+    double kb[2][8], gs[2][3];
+    for (int q = 0; q < 2; ++q) {
+      for (int i = 0; i < 8; ++i) kb[q][i] = 0.0;
+      for (int v = 0; v < 3; ++v) gs[q][v] = 0.0;
+    }
     for (int qp = 0; qp < 4; ++qp) {
       double g[4][2], w;
       quad4_point(x, qp, g, &w);
-      double ga[2] = {g[0][0], g[0][1]};
-#pragma unroll
-      for (int n = 1; n < 4; ++n)
-        if (la == n) { ga[0] = g[n][0]; ga[1] = g[n][1]; }
-#pragma unroll
       for (int q = 0; q < 2; ++q) {
         double part[3];
-        bt_d_row<2, double>(D, ga, q, part);
-#pragma unroll
+        bt_d_row<2, double>(D, g[la], q, part);
         for (int b = 0; b < 4; ++b)
-#pragma unroll
-          for (int q2 = 0; q2 < 2; ++q2) kb[b][q * 2 + q2] += w * part_b<2, double>(part, g[b], q2);
+          for (int q2 = 0; q2 < 2; ++q2) kb[q][b * 2 + q2] += w * part_b<2, double>(part, g[b], q2);
+        for (int v = 0; v < 3; ++v) gs[q][v] += w * part[v];
       }
-      double eps[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int n = 0; n < 4; ++n) add_strain<2, double>(g[n], u[n], eps);
-      if (P.subscale) {
-#pragma unroll
-        for (int v = 0; v < 3; ++v) eps[v] += P.eps_macro[v];
-      }
-      double sig[3];
-      lei_stress<2, double>(D, eps, sig);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) r[q] += w * bt_sig<2, double>(ga, sig, q);
     }
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) blk[b * D2 + i] = kb[b][i];
-    rv[0] = r[0];
-    rv[1] = r[1];
+    for (int q = 0; q < 2; ++q) {
+      for (int i = 0; i < 8; ++i) blk[q * pitch + i] += kb[q][i];
+      for (int v = 0; v < 3; ++v) G[q * 3 + v] += gs[q][v];
+    }
   } else {
-    double x[NPE][DIM], g[NPE][DIM], J;
-#pragma unroll
-    for (int n = 0; n < NPE; ++n) load_node<DIM>(P.X, nd[n], x[n]);
+    double g[NPE][DIM], J;
     simplex_geom<DIM, double>(x, g, &J);
     const double wgt = J * ((DIM == 2) ? tri4_wsum() : tet5_wsum());
-    double ga[DIM];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) ga[d] = g[0][d];
-#pragma unroll
-    for (int n = 1; n < NPE; ++n)
-      if (la == n)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) ga[d] = g[n][d];
-#pragma unroll
     for (int q = 0; q < DIM; ++q) {
       double part[NV];
-      bt_d_row<DIM, double>(D, ga, q, part);
-#pragma unroll
+      bt_d_row<DIM, double>(D, g[la], q, part);
       for (int b = 0; b < NPE; ++b)
-#pragma unroll
-        for (int q2 = 0; q2 < DIM; ++q2) blk[b * D2 + q * DIM + q2] = wgt * part_b<DIM, double>(part, g[b], q2);
-    }
-    double eps[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) eps[v] = 0.0;
-#pragma unroll
-    for (int n = 0; n < NPE; ++n) {
-      double u[DIM];
-      load_node<DIM>(P.U, nd[n], u);
-      add_strain<DIM, double>(g[n], u, eps);
-    }
-    if (P.subscale) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) eps[v] += P.eps_macro[v];
-    }
-    double sig[NV];
-    lei_stress<DIM, double>(D, eps, sig);
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) rv[q] = wgt * bt_sig<DIM, double>(ga, sig, q);
-  }
-}
-
-// Static residual of a general node next to cut elements: sum over its neighbour slots (in slot
-// order) of the static block times the slot node's displacement, then the macroscale-strain
-// response.  `part` holds the per-slot products (slot-major, DIM each), written by the caller's
-// lanes; the sum runs on one lane, so it does not depend on how many lanes formed the products.
-template <int DIM>
-__device__ __forceinline__ void static_resid_sum(const DevProblem& P, int node, int nn, const double* part,
-                                                 const double* eps, double* r) {
-  constexpr int NV = (DIM == 2) ? 3 : 6;
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) r[q] = 0.0;
-  for (int k = 0; k < nn; ++k)
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) r[q] += part[k * DIM + q];
-  if (P.subscale) {
-    const double* Gs = P.stat_g + (size_t)node * DIM * NV;
-#pragma unroll
-    for (int q = 0; q < DIM; ++q)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) r[q] += __ldg(&Gs[q * NV + v]) * eps[v];
-  }
-}
-
-// Product of static slot k of a general node with the slot node's displacement (one slot's
-// contribution to the static residual).
-template <int DIM>
-__device__ __forceinline__ void static_slot_product(const DevProblem& P, int s0, int k, double* out) {
-  constexpr int D2 = DIM * DIM;
-  const double* S = P.stat + (size_t)(s0 + k) * D2;
-  double u[DIM];
-  load_node<DIM>(P.U, __ldg(&P.stat_node[s0 + k]), u);
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) {
-    double v = 0.0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) v += __ldg(&S[q * DIM + d]) * u[d];
-    out[q] = v;
-  }
-}
-
-// The cohesive element's block (n1, n2) and the traction at n1 for a row node at cohesive place
-// cpa = (element << 5 | n1): sgn * B_{n1 % nh, n2 % nh} and sgn * t_{n1 % nh}
-// (cohesiveKFast / cohesiveInternalForceFast signs).
-template <int DIM>
-__device__ __forceinline__ void coh_block_add(const DevProblem& P, int cpa, int cpb, double* blk) {
-  constexpr int D2 = DIM * DIM;
-  const int ce = cpa >> 5, n1 = cpa & 31, n2 = cpb & 31;
-  const int nh = __ldg(&P.coh_nh[ce]);
-  const double sgn = ((n1 >= nh) == (n2 >= nh)) ? 1.0 : -1.0;
-  const double* B = P.kcoh + __ldg(&P.kc_off[ce]) + ((n1 % nh) * nh + (n2 % nh)) * D2;
-#pragma unroll
-  for (int i = 0; i < D2; ++i) blk[i] = sgn * B[i];
-}
-template <int DIM>
-__device__ __forceinline__ void coh_traction(const DevProblem& P, int cpa, double* t) {
-  constexpr int D2 = DIM * DIM;
-  const int ce = cpa >> 5, n1 = cpa & 31;
-  const int nh = __ldg(&P.coh_nh[ce]);
-  const double sgn = (n1 >= nh) ? 1.0 : -1.0;
-  const double* tp = P.kcoh + __ldg(&P.kc_off[ce]) + nh * nh * D2 + (n1 % nh) * DIM;
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) t[q] = sgn * tp[q];
-}
-
-// Row assembly for the DOF nodes the stencil path does not take (boundary rows, nodes of cut
-// elements, enrichment nodes): one lane group of L threads per DOF node, its rows in a
-// shared-memory slab.  The slab starts from the node's static part (the cut elements' volumetric
-// blocks summed per neighbour slot at set-up; zero for nodes without cut elements) and the
-// residual from the static blocks times the displacements plus the macroscale-strain response.
-// The node's adjacent elements then follow in adjacency order (cut elements first):
-//   * a cut element the row node is on a cohesive element of adds that cohesive element's blocks
-//     and traction (k_coh_elements left them in kcoh), its lanes taking the element's nodes;
-//   * the uncut elements are taken L at a time: lane k recomputes element e0 + k from the node
-//     coordinates and writes its whole block row and residual to its scratch record, then the
-//     lanes add the records into the slab in entry order, each lane owning the slots s = k,
-//     k + L, ... (an element's nodes have distinct slots), and lane 0 adds the residuals.
-// Every sum therefore runs in a fixed order that does not depend on L.  Finally the group writes
-// every CSR value of the node's rows exactly once.
-//   gdesc[node]      int4 {adjacency begin, adjacency count, neighbour begin, neighbour count}
-//   growd[node]      3*DIM ints: global DOF of each row, first slot in the row's F block, in its C block
-//   adesc[entry]     int4 {element, local node | nodes of a cut element << 8, slots (uncut: 8 bits per
-//                    node; cut: offset into adj_slots), material (uncut)}
-//   aresd[entry]     int4: uncut {element nodes (-1 padded)}; cut {cut element, its first node in
-//                    cut_nodes, the row node's cohesive place (element << 5 | position) or -1, 0}
-//   nbr_pre[slot]    free DOFs of the node's neighbours before this one (row positions)
-// `valid` is uniform over the group, and the group synchronises only its own lanes.  `slab` is the
-// group's general_slab_doubles(slab_slots, DIM, L) doubles.  (Residual-only assemblies use
-// k_rows_general_resid.)
-template <int DIM, int L, int NPE = DIM + 1>
-__device__ __forceinline__ void general_rows(const DevProblem& P, int node, bool valid, double* slab, int slab_slots) {
-  constexpr int D2 = DIM * DIM;
-  constexpr int LD = general_lane_doubles(DIM, NPE);
-  if (!valid) return;
-  const int g = threadIdx.x % L;
-  const unsigned gmask = (L >= 32) ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x & 31) / L * L));
-  const int4 gd = __ldg(&P.gdesc[node]);
-  const int nn = gd.w;
-  const bool stat = node < P.n_stat;
-  double* rs = slab + nn * D2;             // residual of the node's rows
-  double* part = rs + 4;                   // per-slot residual partials of the static part
-  double* scr = slab + general_scratch_offset(slab_slots, DIM);
-  if (stat) {
-    const int s0 = __ldg(&P.stat_slot_off[node]);
-    const double* S = P.stat + (size_t)s0 * D2;
-    for (int i = g; i < nn * D2; i += L) slab[i] = __ldg(&S[i]);
-    for (int k = g; k < nn; k += L) static_slot_product<DIM>(P, s0, k, part + k * DIM);
-  } else {
-    for (int i = g; i < nn * D2; i += L) slab[i] = 0.0;
-  }
-  __syncwarp(gmask);
-  if (g == 0) {
-    double r[DIM];
-    if (stat) static_resid_sum<DIM>(P, node, nn, part, P.eps_macro, r);
-    else
-#pragma unroll
-      for (int q = 0; q < DIM; ++q) r[q] = 0.0;
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) rs[q] = r[q];
-  }
-  __syncwarp(gmask);
-  // cut entries (first in the adjacency order): the cohesive element the row node is on
-  int e = 0;
-  for (; e < gd.y; ++e) {
-    const int4 ad = __ldg(&P.adesc[gd.x + e]);
-    const int mn = ad.y >> 8;
-    if (mn == 0) break;
-    const int4 ax = __ldg(&P.aresd[gd.x + e]);
-    const int cpa = ax.z;
-    if (cpa < 0) continue;
-    for (int b = g; b < mn; b += L) {
-      const int cpb = __ldg(&P.cohpos[ax.y + b]);
-      if (cpb >= 0 && (cpb >> 5) == (cpa >> 5)) {
-        double blk[D2];
-        coh_block_add<DIM>(P, cpa, cpb, blk);
-        slab_add<DIM>(slab + __ldg(&P.adj_slots[ad.z + b]) * D2, blk);
-      }
-    }
-    if (g == 0) {
-      double t[DIM];
-      coh_traction<DIM>(P, cpa, t);
-#pragma unroll
-      for (int q = 0; q < DIM; ++q) rs[q] += t[q];
-    }
-    __syncwarp(gmask);
-  }
-  // uncut entries, L at a time
-  for (int e0 = e; e0 < gd.y; e0 += L) {
-    double* my = scr + g * LD;
-    unsigned z = 0u;
-    if (e0 + g < gd.y) {
-      const int4 ad = __ldg(&P.adesc[gd.x + e0 + g]);
-      const int4 ax = __ldg(&P.aresd[gd.x + e0 + g]);
-      uncut_block_row<DIM, NPE>(P, ax, ad.y & 255, P.D[ad.w], my, my + NPE * D2);
-      z = (unsigned)ad.z;
-    }
-    reinterpret_cast<unsigned*>(my + NPE * D2 + DIM)[0] = z;
-    __syncwarp(gmask);
-    const int n_here = min(L, gd.y - e0);
-    for (int s = g; s < nn; s += L) {
-      double acc[D2];
-#pragma unroll
-      for (int i = 0; i < D2; ++i) acc[i] = slab[s * D2 + i];
-      for (int j = 0; j < n_here; ++j) {
-        const double* oj = scr + j * LD;
-        const unsigned zj = reinterpret_cast<const unsigned*>(oj + NPE * D2 + DIM)[0];
-#pragma unroll
-        for (int b = 0; b < NPE; ++b)
-          if (((zj >> (8 * b)) & 255u) == (unsigned)s)
-#pragma unroll
-            for (int i = 0; i < D2; ++i) acc[i] += oj[b * D2 + i];
-      }
-#pragma unroll
-      for (int i = 0; i < D2; ++i) slab[s * D2 + i] = acc[i];
-    }
-    if (g == 0)
-      for (int j = 0; j < n_here; ++j)
-#pragma unroll
-        for (int q = 0; q < DIM; ++q) rs[q] += scr[j * LD + NPE * D2 + q];
-    __syncwarp(gmask);
-  }
-  const uint8_t* masks = P.dn_nbr_mask + gd.z;
-  const int* pre = P.nbr_pre + gd.z;
-  const int* rd = P.growd + (size_t)node * 3 * DIM;
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) {
-    const int gdof = __ldg(&rd[q]);
-    const bool rf = gdof < P.n_free;
-    if (P.flags & FLAG_JAC) {
-      double* vF = P.val[rf ? 0 : 2] + __ldg(&rd[DIM + q]);
-      double* vC = P.val[rf ? 1 : 3] + __ldg(&rd[2 * DIM + q]);
-      for (int k = g; k < nn; k += L) {
-        int pf = __ldg(&pre[k]);
-        int pc = k * DIM - pf;
-        const int mk = __ldg(&masks[k]);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          const double v = slab[(k * DIM + q) * DIM + d];
-          if (mk & (1 << d)) vF[pf++] = v; else vC[pc++] = v;
-        }
-      }
-    }
-    if ((P.flags & FLAG_FUNC) && g == 0) {
-      if (rf) P.Pf[gdof] = rs[q]; else P.Pp[gdof - P.n_free] = rs[q];
+        for (int q2 = 0; q2 < DIM; ++q2) blk[q * pitch + b * DIM + q2] += wgt * part_b<DIM, double>(part, g[b], q2);
+      for (int v = 0; v < NV; ++v) G[q * NV + v] += wgt * part[v];
     }
   }
 }
 
-// Static residual of a general node for a group of L lanes (lane k of the group): the per-slot
-// products of static_slot_product summed in slot order with shuffles, as static_resid_sum sums
-// them, without the macroscale-strain response.  Every lane of the group gets the sum.
-template <int DIM, int L>
-__device__ __forceinline__ void static_resid_group(const DevProblem& P, int node, int nn, int k, unsigned gmask,
-                                                   double* r) {
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) r[q] = 0.0;
-  const int s0 = __ldg(&P.stat_slot_off[node]);
-  for (int k0 = 0; k0 < nn; k0 += L) {           // nn is uniform over the group
-    double pk[DIM];
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) pk[q] = 0.0;
-    if (k0 + k < nn) static_slot_product<DIM>(P, s0, k0 + k, pk);
-    const int n_here = min(L, nn - k0);
-    for (int j = 0; j < n_here; ++j)
-#pragma unroll
-      for (int q = 0; q < DIM; ++q) r[q] += __shfl_sync(gmask, pk[q], j, L);
-  }
-}
-
-// Residual-only rows of the general nodes, entry-parallel: L lanes per DOF node.  The node's
-// static residual first (static blocks times displacements in slot order, then the macroscale-
-// strain response), then lane k takes the node's entries k, k + L, ... and forms each entry's
-// contribution (an uncut element's w B^T sigma; the cohesive traction at the node for a cut
-// element the node is on a cohesive element of) -- the same operations general_rows performs --
-// and the group adds the contributions in entry (adjacency) order with shuffles.  L divides 32.
-template <int DIM, int L, int NPE = DIM + 1>
-__global__ void __launch_bounds__(128) k_rows_general_resid(DevProblem P) {
-  constexpr int NV = (DIM == 2) ? 3 : 6;
-  constexpr int D2 = DIM * DIM;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int node = t / L, k = t % L;
-  const bool valid = node < P.n_slow_dn;   // uniform over each group of L lanes
-  const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x & 31) / L * L));
-  if (__all_sync(0xffffffffu, !valid)) return;
-  int4 gd = make_int4(0, 0, 0, 0);
-  if (valid) gd = __ldg(&P.gdesc[node]);
-  double rs[DIM];
-#pragma unroll
-  for (int q = 0; q < DIM; ++q) rs[q] = 0.0;
-  if (valid && node < P.n_stat) {                // uniform over the group
-    static_resid_group<DIM, L>(P, node, gd.w, k, gmask, rs);
-    if (P.subscale) {
-      const double* Gs = P.stat_g + (size_t)node * DIM * NV;
-#pragma unroll
-      for (int q = 0; q < DIM; ++q)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) rs[q] += __ldg(&Gs[q * NV + v]) * P.eps_macro[v];
-    }
-  }
-  for (int e0 = 0; e0 < gd.y; e0 += L) {          // gd.y is uniform over the group
-    const int ei = e0 + k;
-    double re[DIM];
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) re[q] = 0.0;
-    if (ei < gd.y) {
-      const int4 ad = __ldg(&P.adesc[gd.x + ei]);
-      const int4 ax = __ldg(&P.aresd[gd.x + ei]);
-      const int la = ad.y & 255, mn = ad.y >> 8;
-      if (mn == 0) {
-        double blk[NPE * D2];   // unused: the stiffness products are left to the compiler to drop
-        uncut_block_row<DIM, NPE>(P, ax, la, P.D[ad.w], blk, re);
-      } else if (ax.z >= 0) {
-        coh_traction<DIM>(P, ax.z, re);
-      }
-    }
-    // the node's sum in entry order
-    const int n_here = min(L, gd.y - e0);
-    for (int j = 0; j < n_here; ++j)
-#pragma unroll
-      for (int q = 0; q < DIM; ++q) rs[q] += __shfl_sync(gmask, re[q], j, L);
-  }
-  if (!valid || k >= DIM || !(P.flags & FLAG_FUNC)) return;
-  double mine = rs[0];
-#pragma unroll
-  for (int q = 1; q < DIM; ++q) if (k == q) mine = rs[q];
-  const int gdof = __ldg(&P.growd[(size_t)node * 3 * DIM + k]);
-  if (gdof < P.n_free) P.Pf[gdof] = mine; else P.Pp[gdof - P.n_free] = mine;
-}
-
-// Set-up: the static part of the general rows (one thread per node of the image): each cut
-// entry's volumetric block row (K_vol, from k_cut_volumetric) added into the node's neighbour
-// slots and its macroscale-strain response into the node's sum, in entry order; in tri3 / tet4
-// meshes the uncut elements' block rows and responses follow (every bulk law is linear elastic,
-// so they do not depend on the state either), while quad4 meshes stop at the first uncut entry
-// (the entries are cut-first).  stat and stat_g start at zero.
+// Set-up: the static image of the general rows, one thread per node: each adjacent element's block
+// row (a cut element's from its volumetric matrix K_vol, k_cut_volumetric; an uncut one's formed
+// here) added into the node's rows, and its macroscale-strain response into the node's sum, in
+// entry order (cut elements first).  A node's image is laid out like its CSR rows: row q at q * (DIM
+// x slots), slot s's columns at s * DIM.  stat and stat_g start at zero.
 template <int DIM>
 __global__ void __launch_bounds__(128) k_general_static(DevProblem P, double* stat, double* stat_g) {
   constexpr int NV = (DIM == 2) ? 3 : 6;
   constexpr int D2 = DIM * DIM;
   const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= P.n_stat) return;
+  if (node >= P.n_slow_dn) return;
   const int4 gd = __ldg(&P.gdesc[node]);
-  double* S = stat + (size_t)__ldg(&P.stat_slot_off[node]) * D2;
+  const int pitch = gd.w * DIM;
+  double* S = stat + (size_t)__ldg(&P.gnd[2 * node]).x * D2;
   double* Gs = stat_g + (size_t)node * DIM * NV;
   bool bad = false;
   for (int e = 0; e < gd.y; ++e) {
@@ -646,52 +215,34 @@ __global__ void __launch_bounds__(128) k_general_static(DevProblem P, double* st
     const int4 ax = __ldg(&P.aresd[gd.x + e]);
     const int la = ad.y & 255, mn = ad.y >> 8;
     if (mn == 0) {
-      // uncut simplex (tri3 / tet4 meshes: every general node's image holds its uncut elements
-      // too): the block row la, w B_la^T D B_b for each element node b, and the macroscale
-      // response w B_la^T D -- the products of simplex_block, once per mesh
-      if (P.npe != DIM + 1) break;
-      constexpr int NPE = DIM + 1;
       const int nd[4] = {ax.x, ax.y, ax.z, ax.w};
-      double x[NPE][DIM], g[NPE][DIM], J;
-      for (int n = 0; n < NPE; ++n) load_node<DIM>(P.X, nd[n], x[n]);
-      simplex_geom<DIM, double>(x, g, &J);
-      const double wgt = J * ((DIM == 2) ? tri4_wsum() : tet5_wsum());
-      const double* D = P.Dd + ad.w * 36;
-      for (int q = 0; q < DIM; ++q) {
-        double part[NV];
-        bt_d_row<DIM, double>(D, g[la], q, part);
-        for (int b = 0; b < NPE; ++b) {
-          double* o = S + (size_t)((ad.z >> (8 * b)) & 255) * D2;
-          for (int q2 = 0; q2 < DIM; ++q2) o[q * DIM + q2] += wgt * part_b<DIM, double>(part, g[b], q2);
-        }
-        for (int v = 0; v < NV; ++v) Gs[q * NV + v] += wgt * part[v];
-      }
+      auto add = [&](auto npe) {
+        constexpr int NPE = decltype(npe)::value;
+        double x[NPE][DIM], blk[DIM * NPE * DIM];
+        for (int n = 0; n < NPE; ++n) load_node<DIM>(P.X, nd[n], x[n]);
+        for (int i = 0; i < DIM * NPE * DIM; ++i) blk[i] = 0.0;
+        element_rows<DIM, NPE>(x, la, P.Dd + ad.w * 36, blk, NPE * DIM, Gs);
+        for (int q = 0; q < DIM; ++q)
+          for (int b = 0; b < NPE; ++b)
+            for (int d = 0; d < DIM; ++d) S[q * pitch + ((ad.z >> (8 * b)) & 255) * DIM + d] += blk[(q * NPE + b) * DIM + d];
+      };
+      if (DIM == 2 && P.npe == 4) { if constexpr (DIM == 2) add(IntC<4>{}); }
+      else add(IntC<DIM + 1>{});
       continue;
     }
     const int cc = ax.x;
     const double* kr = P.ke + __ldg(&P.ke_off[cc]) + (size_t)la * mn * D2;   // block row la of K_vol
     for (int b = 0; b < mn; ++b) {
-      double* o = S + (size_t)__ldg(&P.adj_slots[ad.z + b]) * D2;
-#pragma unroll
-      for (int i = 0; i < D2; ++i) o[i] += kr[b * D2 + i];
+      double* o = S + __ldg(&P.adj_slots[ad.z + b]) * DIM;
+      for (int q = 0; q < DIM; ++q)
+        for (int d = 0; d < DIM; ++d) o[q * pitch + d] += kr[b * D2 + q * DIM + d];
     }
     const double* gm = P.gmac + (size_t)__ldg(&P.re_off[cc]) / DIM * DIM * NV + (size_t)la * DIM * NV;
 #pragma unroll
     for (int i = 0; i < DIM * NV; ++i) Gs[i] += gm[i];
   }
-  for (int i = 0; i < gd.w * D2; ++i) bad |= !isfinite(S[i]);
+  for (int i = 0; i < pitch * DIM; ++i) bad |= !isfinite(S[i]);
   if (bad) atomicOr(P.err, ERR_NONFINITE);
-}
-
-// General rows of the nodes [node0, node1) of the general list.
-template <int DIM, int L, int NPE = DIM + 1>
-__global__ void __launch_bounds__(128) k_rows_general(DevProblem P, int slab_slots, int node0, int node1) {
-  constexpr int NB = 128 / L;
-  extern __shared__ double smem[];
-  const int grp = threadIdx.x / L;
-  const int node = node0 + blockIdx.x * NB + grp;
-  general_rows<DIM, L, NPE>(P, node, node < node1,
-                            smem + (size_t)grp * general_slab_doubles(slab_slots, DIM, L, NPE), slab_slots);
 }
 
 // Cohesive elements, one lane per quadrature point (CQ lanes per element: 2 in 2D for CohEdge2, 4
@@ -826,14 +377,6 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
 #pragma unroll
     for (int i = 0; i < DIM; ++i) out[nh * nh * D2 + a * DIM + i] = t[i];
   }
-}
-
-template <int DIM>
-__global__ void __launch_bounds__(128) k_coh_elements(DevProblem P) {
-  constexpr int CQ = CohLanes<DIM>::CQ;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ce = t / CQ;
-  coh_element<DIM>(P, ce, t % CQ, ce < P.n_coh_el);
 }
 
 // State-independent part of the cut elements, computed once at set-up: the volumetric element

@@ -12,6 +12,7 @@
 //                  (Problem::homogenize, src/Problem.cpp:471-484, with the stress functor of
 //                  include/AssemblerSmallStrainStructural.h:31-60).
 #include "pg_ctx.h"
+#include "pg_kernels.cuh"
 
 #include <algorithm>
 #include <cmath>
