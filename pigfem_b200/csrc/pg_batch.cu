@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(pgd::kRowThreads) k_batch_coh(const pgd::DevPr
 }
 
 // item = {context, part, block of the part, -}
-template <int DIM>
+template <int DIM, bool JAC>
 __global__ void __launch_bounds__(pgd::kRowThreads) k_batch_rows(const pgd::DevProblem* __restrict__ items, const BatchCall* call,
                                                                  const int4* __restrict__ list, int n, int* err) {
   __shared__ pgd::DevProblem view;
@@ -74,8 +74,7 @@ __global__ void __launch_bounds__(pgd::kRowThreads) k_batch_rows(const pgd::DevP
     if (it.x != last) load_view(view, items, call, it.x, err);
     last = it.x;
     if (it.y == 1 && !(view.flags & pgd::FLAG_FUNC)) continue;
-    if (it.y == 3 && !(view.flags & pgd::FLAG_JAC)) continue;
-    pgd::row_block<DIM, pgd::pattern_period(DIM, DIM + 1), false>(view, it.y, it.z);
+    pgd::row_block<DIM, pgd::pattern_period(DIM, DIM + 1), false, JAC, true>(view, it.y, it.z);
   }
 }
 
@@ -93,7 +92,7 @@ struct pg_batch {
   int mult = 4;   // launch shape (autotuned): persistent blocks per SM
   cudaStream_t stream = nullptr;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraphExec_t exec[2] = {nullptr, nullptr};   // residuals only, with the matrices
   bool launched = false;
   long long n_elem = 0;
   std::string err;
@@ -113,8 +112,8 @@ void free_lists(pg_batch* b) {
 }
 
 void drop_graphs(pg_batch* b) {
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  b->exec = nullptr;
+  for (auto& e : b->exec)
+    if (e) { cudaGraphExecDestroy(e); e = nullptr; }
 }
 
 template <typename T>
@@ -131,26 +130,33 @@ int upload_vec(pg_batch* b, const std::vector<T>& h, T** d) {
 int build_lists(pg_batch* b) {
   free_lists(b);
   drop_graphs(b);
-  // the general rows first and the CSR chunks last, as in a single assembly
+  // the rows' blocks of all contexts, mixed as in a single assembly
   std::vector<int4> coh, rows;
-  b->n_sten = b->n_gen = 0;
   const int per = pgd::kRowThreads / ((b->dim == 2) ? pgd::CohLanes<2>::CQ : pgd::CohLanes<3>::CQ);
-  for (int part = 0; part < 4; ++part)
-    for (int i = 0; i < (int)b->ctx.size(); ++i) {
-      const pgd::DevProblem& P = b->ctx[i]->P;
-      const int n = pgd::row_parts(P, true, true, false).n[part];
-      for (int k = 0; k < n; ++k) rows.push_back(make_int4(i, part, k, 0));
-      ((part & 1) ? b->n_sten : b->n_gen) += n;
-      if (part == 0)
-        for (int f = 0; f < P.n_coh_el; f += per) coh.push_back(make_int4(i, f, 0, 0));
-    }
+  std::vector<int4> of[4];
+  pgd::RowParts all = {{0, 0, 0, 0}, false, 0};
+  for (int i = 0; i < (int)b->ctx.size(); ++i) {
+    const pgd::DevProblem& P = b->ctx[i]->P;
+    const pgd::RowParts p = pgd::row_parts(P, true, true, false);
+    for (int part = 0; part < 4; ++part)
+      for (int k = 0; k < p.n[part]; ++k, ++all.n[part]) of[part].push_back(make_int4(i, part, k, 0));
+    for (int f = 0; f < P.n_coh_el; f += per) coh.push_back(make_int4(i, f, 0, 0));
+  }
+  all.spread();
+  for (int k = 0; k < all.total(); ++k) {
+    int part, item;
+    all.pick(k, &part, &item);
+    rows.push_back(of[part][item]);
+  }
+  b->n_sten = all.n[1] + all.n[3];
+  b->n_gen = all.n[0] + all.n[2];
   b->n_coh = (int)coh.size();
   int rc = upload_vec(b, coh, &b->d_coh);
   return rc ? rc : upload_vec(b, rows, &b->d_rows);
 }
 
 template <int DIM>
-void enqueue_dim(pg_batch* b) {
+void enqueue_dim(pg_batch* b, bool jac) {
   cudaStream_t st = b->stream;
   const int cap = b->mult * kSMs, n_rows = b->n_sten + b->n_gen;
   if (b->n_coh)
@@ -165,26 +171,26 @@ void enqueue_dim(pg_batch* b) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = b->n_coh ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k_batch_rows<DIM>, (const pgd::DevProblem*)b->d_items, (const BatchCall*)b->d_call, (const int4*)b->d_rows,
-                     n_rows, b->d_err);
+  cudaLaunchKernelEx(&cfg, jac ? k_batch_rows<DIM, true> : k_batch_rows<DIM, false>, (const pgd::DevProblem*)b->d_items,
+                     (const BatchCall*)b->d_call, (const int4*)b->d_rows, n_rows, b->d_err);
 }
 
-void enqueue(pg_batch* b) {
+void enqueue(pg_batch* b, bool jac) {
   cudaStream_t st = b->stream;
   cudaMemcpyAsync(b->d_call, b->h_call, sizeof(BatchCall) * b->ctx.size(), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(b->d_err, 0, sizeof(int), st);
-  if (b->dim == 2) enqueue_dim<2>(b);
-  else enqueue_dim<3>(b);
+  if (b->dim == 2) enqueue_dim<2>(b, jac);
+  else enqueue_dim<3>(b, jac);
   cudaMemcpyAsync(b->h_err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
 }
 
-int graph_for(pg_batch* b, cudaGraphExec_t* out) {
-  cudaGraphExec_t& e = b->exec;
+int graph_for(pg_batch* b, bool jac, cudaGraphExec_t* out) {
+  cudaGraphExec_t& e = b->exec[jac ? 1 : 0];
   if (!e) {
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return berr(b, PG_ERR_DEVICE, "graph capture failed to start");
-    enqueue(b);
+    enqueue(b, jac);
     if (cudaStreamEndCapture(b->stream, &g) != cudaSuccess) return berr(b, PG_ERR_DEVICE, "graph capture failed");
     const cudaError_t ie = cudaGraphInstantiate(&e, g, 0);
     cudaGraphDestroy(g);
@@ -246,7 +252,7 @@ int pg_batch_assemble(pg_batch* b, const double* const* d_U, const double* t_fra
   }
   fill_call(b, d_U, t_frac, flags);
   cudaGraphExec_t e;
-  if (int rc = graph_for(b, &e)) return rc;
+  if (int rc = graph_for(b, (flags & PG_JAC) != 0, &e)) return rc;
   cudaEventRecord(b->t0, b->stream);
   if (cudaGraphLaunch(e, b->stream) != cudaSuccess) return berr(b, PG_ERR_DEVICE, "graph launch failed");
   cudaEventRecord(b->t1, b->stream);

@@ -37,27 +37,50 @@ int dalloc(pg_ctx* c, size_t n, T** out) { return pg_dalloc(c, n, out); }
 
 #define PG_TRY(x) do { int _e = (x); if (_e) return _e; } while (0)
 
-// Fixed-order sum of squares: each block reduces a contiguous chunk in a fixed tree order.
-__global__ void k_sumsq_partial(const double* x, int n, double* part) {
-  __shared__ double sh[256];
-  const int chunk = (n + gridDim.x - 1) / gridDim.x;
-  const int b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
-  double s = 0.0;
-  for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) s += x[i] * x[i];
-  sh[threadIdx.x] = s;
+// Fixed-order sum of squares in one launch: block b reduces the values [b, b + 1) * kNormBlock with a
+// fixed tree into part[b]; the block that finishes last sums the partials in block order and writes
+// the root to pinned host memory.  Small systems take one block.  (Two launches, a serial sum over
+// 256 partials by one thread and a copy took 17 us for 3,000 rows.)
+constexpr int kNormThreads = 512, kNormBlock = 8 * kNormThreads;
+__device__ __forceinline__ double block_total(double s, double* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+  s = (threadIdx.x < kNormThreads / 32) ? sh[threadIdx.x] : 0.0;
+  if (threadIdx.x < 32)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;   // in thread 0
 }
-__global__ void k_sum_final(const double* part, int n, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    out[0] = s;
+__global__ void __launch_bounds__(kNormThreads) k_norm(const double* __restrict__ x, int n, double* part, unsigned* count, double* out) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  const long long b0 = (long long)blockIdx.x * kNormBlock;
+  double v[8], s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const long long i = b0 + k * kNormThreads + threadIdx.x;
+    v[k] = (i < n) ? x[i] : 0.0;
   }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = __fma_rn(v[k], v[k], s);
+  s = block_total(s, sh);
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) {
+      part[blockIdx.x] = s;
+      __threadfence();
+      last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kNormThreads) s += __ldcg(&part[i]);
+    s = block_total(s, sh);
+    if (threadIdx.x == 0) *count = 0;   // ready for the next call on the stream
+  }
+  if (threadIdx.x == 0) *out = sqrt(s);
 }
 
 // The structured rows' constants (pg_rows.cuh): the shapes' element matrices (k_shape_consts) summed
@@ -508,24 +531,7 @@ int pg_upload(pg_ctx* c) {
     PG_TRY(upload(c, dg_off, &P.qp_grad_off));
     PG_TRY(upload(c, dg, &P.qp_grad));
   }
-  PG_TRY(upload(c, s.cut_coh_off, &P.cut_coh_off));
-  PG_TRY(upload(c, s.coh_nh, &P.coh_nh));
-  PG_TRY(upload(c, s.coh_local_off, &P.coh_local_off));
-  PG_TRY(upload(c, s.coh_local, &P.coh_local));
-  PG_TRY(upload(c, s.coh_qp_off, &P.coh_qp_off));
   PG_TRY(upload(c, s.cqp_N, &P.cqp_N));
-  {
-    std::vector<int> noff;
-    noff.reserve(s.cqp_wgt.size() + 1);
-    for (size_t ce = 0; ce + 1 < s.coh_qp_off.size(); ++ce)
-      for (int cq = s.coh_qp_off[ce]; cq < s.coh_qp_off[ce + 1]; ++cq) noff.push_back(0);
-    // running offsets: each point of cohesive element ce holds coh_nh[ce] shape values
-    int o = 0, k = 0;
-    for (size_t ce = 0; ce + 1 < s.coh_qp_off.size(); ++ce)
-      for (int cq = s.coh_qp_off[ce]; cq < s.coh_qp_off[ce + 1]; ++cq) { noff[k++] = o; o += s.coh_nh[ce]; }
-    if (o != (int)s.cqp_N.size()) return set_err(c, PG_ERR_STATE, "internal: cohesive shape-value count mismatch");
-    PG_TRY(upload(c, noff, &P.cqp_noff));
-  }
   PG_TRY(upload(c, s.cqp_R, &P.cqp_R));
   PG_TRY(upload(c, s.cqp_wgt, &P.cqp_wgt));
   PG_TRY(upload(c, s.cqp_isv, &P.cqp_isv));
@@ -581,7 +587,18 @@ int pg_upload(pg_ctx* c) {
           gnode[k] = s.cut_nodes[s.cut_node_off[ce_cut[ce]] + s.coh_local[k]];
       PG_TRY(upload(c, gnode, &P.coh_gnode));
     }
-    PG_TRY(upload(c, kc_off, &P.kc_off));
+    {
+      std::vector<int4> cdesc;
+      int o = 0;
+      for (int ce = 0; ce < n_ce; ++ce) {
+        const int nh = s.coh_nh[ce], nq = s.coh_qp_off[ce + 1] - s.coh_qp_off[ce];
+        cdesc.push_back(make_int4(s.coh_local_off[ce], s.coh_qp_off[ce], o, kc_off[ce]));
+        cdesc.push_back(make_int4(nh, nq, 0, 0));
+        o += nh * nq;
+      }
+      if (o != (int)s.cqp_N.size()) return set_err(c, PG_ERR_STATE, "internal: cohesive shape-value count mismatch");
+      PG_TRY(upload(c, cdesc, &P.cdesc));
+    }
     kc_off_h = kc_off;
     cohpos_h = cohpos;
     double* dk;
@@ -632,7 +649,7 @@ int pg_upload(pg_ctx* c) {
   PG_TRY(dalloc(c, (size_t)n_nodes * dim, &c->d_U));
   PG_TRY(dalloc(c, 1, &c->d_err));
   P.err = c->d_err;
-  PG_TRY(dalloc(c, 1024, &c->d_red));
+  PG_TRY(dalloc(c, 2 + (size_t)s.n_free / kNormBlock + 1, &c->d_red));
   // Static image of the general rows (k_general_static), the node ids of its slots, the cohesive
   // contributions of every slot in adjacency order and the nodes' traction lists
   {
@@ -768,6 +785,7 @@ void pg_destroy(pg_ctx* c) {
   if (c->pcg.stream) cudaStreamDestroy(c->pcg.stream);
   for (cudaEvent_t e : {c->pcg.ev, c->pcg.evc[0], c->pcg.evc[1]}) if (e) cudaEventDestroy(e);
   if (c->pcg.hflag) cudaFreeHost(c->pcg.hflag);
+  if (c->h_norm) cudaFreeHost(c->h_norm);
   for (cudaEvent_t e : c->ev) if (e) cudaEventDestroy(e);
   for (void* p : c->allocs) cudaFreeAsync(p, c->up);
   if (c->up) cudaStreamDestroy(c->up);   // released once the frees have run
@@ -962,13 +980,12 @@ int pg_set_macro_strain(pg_ctx* c, const double* eps) {
 int pg_residual_norm(pg_ctx* c, double* out) {
   if (!c || !out) return PG_ERR_INPUT;
   if (!pg_resident(c)) return set_err(c, PG_ERR_STATE, "the context has no device residency (pg_upload it first)");
-  const int nb = 256;
-  k_sumsq_partial<<<nb, 256, 0, c->stream>>>(c->P.Pf, c->s.n_free, c->d_red);
-  k_sum_final<<<1, 32, 0, c->stream>>>(c->d_red, nb, c->d_red + nb);
-  double v = 0.0;
-  cudaMemcpyAsync(&v, c->d_red + nb, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+  if (!c->h_norm && cudaMallocHost(&c->h_norm, sizeof(double)) != cudaSuccess)
+    return set_err(c, PG_ERR_DEVICE, "pinned norm allocation failed");
+  const int nb = std::max(1, (int)(((long long)c->s.n_free + kNormBlock - 1) / kNormBlock));
+  k_norm<<<nb, kNormThreads, 0, c->stream>>>(c->P.Pf, c->s.n_free, c->d_red + 1, reinterpret_cast<unsigned*>(c->d_red), c->h_norm);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "residual norm failed");
-  *out = sqrt(v);
+  *out = *c->h_norm;
   return 0;
 }
 

@@ -43,7 +43,8 @@ struct pg_ctx {
   double* d_isv_trial = nullptr;
   uint8_t* d_zone = nullptr;
   int* d_err = nullptr;
-  double* d_red = nullptr;  // residual-norm partials
+  double* d_red = nullptr;  // residual norm: the count of finished blocks, then their partials
+  double* h_norm = nullptr; // its result (pinned host memory the kernel writes)
   long long cut_scratch = 0;   // doubles of the cut elements' set-up blocks (released after set-up)
   int max_nd = 0;
   int n_coh_qp = 0;

@@ -57,9 +57,11 @@ struct DevProblem {
   // cut elements
   const int* cut_node_off; const int* cut_nodes;
   const int* cut_qp_off; const double* qp_wgt; const int* qp_mat; const int* qp_grad_off; const double* qp_grad;
-  const int* cut_coh_off; const int* coh_nh; const int* coh_local_off; const int* coh_local;
-  const int* coh_qp_off; const double* cqp_N; const double* cqp_R; const double* cqp_wgt; const int* cqp_isv;
-  const int* cqp_noff;  // first shape value of each cohesive point in cqp_N (CohTri3 3, CohQuad4 4, CohEdge2 2)
+  const double* cqp_N; const double* cqp_R; const double* cqp_wgt; const int* cqp_isv;
+  // per cohesive element two int4: {its first node in coh_gnode, its first point, the point's first
+  // shape value in cqp_N (nh per point), its first value in kcoh}, {nh (CohEdge2 2, CohTri3 3,
+  // CohQuad4 4), points, -, -}
+  const int4* cdesc;
   const long long* ke_off;  // per cut element: offset of its element matrix in ke
   const int* re_off;        // per cut element: offset of its first node's rows (nodes x dim)
   double* ke;               // set-up only: volumetric element matrices of the cut elements
@@ -98,7 +100,6 @@ struct DevProblem {
   int n_coh_qp;
   int n_coh_el;                                  // cohesive elements
   const int* coh_gnode;                          // node id of every cohesive element's local node ('-' then '+', at coh_local_off)
-  const int* kc_off;                             // per cohesive element: offset of its blocks in kcoh
   double* kcoh;                                  // per call: cohesive blocks B_ab and tractions t_a
   const int* nbr_pre;                            // per neighbour slot: free DOFs of the earlier neighbours
   // outputs: CSR values of the four blocks and the two residual parts

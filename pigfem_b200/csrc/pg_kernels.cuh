@@ -263,12 +263,15 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
   constexpr int D2 = DIM * DIM;
   constexpr int CQ = CohLanes<DIM>::CQ;
   const int lane = threadIdx.x & 31, base_lane = lane & ~(CQ - 1);
-  int nh = 0, q0 = 0, nq = 0;
+  int4 d4 = make_int4(0, 0, 0, 0);
+  int nh = 0, nq = 0;
   if (valid) {
-    nh = __ldg(&P.coh_nh[ce]);
-    q0 = __ldg(&P.coh_qp_off[ce]);
-    nq = min(CQ, __ldg(&P.coh_qp_off[ce + 1]) - q0);
+    d4 = __ldg(&P.cdesc[2 * ce]);
+    const int4 e4 = __ldg(&P.cdesc[2 * ce + 1]);
+    nh = e4.x;
+    nq = min(CQ, e4.y);
   }
+  const int q0 = d4.y;
   double W[D2], Tr[DIM];
 #pragma unroll
   for (int i = 0; i < D2; ++i) W[i] = 0.0;
@@ -276,20 +279,32 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
   for (int i = 0; i < DIM; ++i) Tr[i] = 0.0;
   bool bad = false;
   if (valid && qi < nq) {
-    const int* gn = P.coh_gnode + __ldg(&P.coh_local_off[ce]);   // the element's node ids
+    const int* gn = P.coh_gnode + d4.x;   // the element's node ids
     const int cq = q0 + qi;
-    const double* N = P.cqp_N + __ldg(&P.cqp_noff[cq]);
-    const double* R = P.cqp_R + (size_t)cq * D2;
+    const double* N = P.cqp_N + d4.z + qi * nh;
+    // (every load below depends on the descriptor alone, except U and the internal variables)
+    const int iv = (P.coh.nvar > 0) ? __ldg(&P.cqp_isv[cq]) : 0;
+    const double w = __ldg(&P.cqp_wgt[cq]);
+    double R[D2];
+#pragma unroll
+    for (int i = 0; i < D2; ++i) R[i] = __ldg(&P.cqp_R[(size_t)cq * D2 + i]);
     double d0[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      double s = 0.0;
-      for (int n = 0; n < nh; ++n) {
-        const int np = __ldg(&gn[n + nh]), nm = __ldg(&gn[n]);
-        s += N[n] * (P.U[(size_t)np * DIM + d] - P.U[(size_t)nm * DIM + d]);
-      }
-      d0[d] = s;
-    }
+    for (int d = 0; d < DIM; ++d) d0[d] = 0.0;
+    constexpr int NH = (DIM == 2) ? 2 : 4;   // nodes of a side, at most
+    int np[NH], nm[NH];
+    double Nn[NH], up[NH][DIM], um[NH][DIM];
+#pragma unroll
+    for (int n = 0; n < NH; ++n)
+      if (n < nh) { nm[n] = __ldg(&gn[n]); np[n] = __ldg(&gn[n + nh]); Nn[n] = __ldg(&N[n]); }
+#pragma unroll
+    for (int n = 0; n < NH; ++n)
+      if (n < nh) { load_node<DIM>(P.U, np[n], up[n]); load_node<DIM>(P.U, nm[n], um[n]); }
+#pragma unroll
+    for (int n = 0; n < NH; ++n)
+      if (n < nh)
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) d0[d] += Nn[n] * (up[n][d] - um[n][d]);
     double dl[DIM], T[DIM], Dc[D2];
 #pragma unroll
     for (int i = 0; i < DIM; ++i) {
@@ -298,7 +313,6 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
       for (int j = 0; j < DIM; ++j) s += R[i * DIM + j] * d0[j];
       dl[i] = s;
     }
-    const int iv = __ldg(&P.cqp_isv[cq]);
     double isv[2] = {0.0, 0.0};
     for (int v = 0; v < P.coh.nvar; ++v) isv[v] = P.isv_committed[iv + v];
     uint8_t z;
@@ -315,7 +329,6 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
         for (int j = 0; j < DIM; ++j) s += R[j * DIM + i] * Dc[j * DIM + k];
         RtD[i * DIM + k] = s;
       }
-    const double w = P.cqp_wgt[cq];
 #pragma unroll
     for (int i = 0; i < DIM; ++i)
 #pragma unroll
@@ -346,7 +359,7 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
   }
   if (bad) atomicOr(P.err, ERR_NONFINITE);
   if (!valid) return;
-  double* out = P.kcoh + __ldg(&P.kc_off[ce]);
+  double* out = P.kcoh + d4.w;
   for (int p = qi; p < nh * nh; p += CQ) {
     const int a = p / nh, b = p - a * nh;
     double blk[D2];
@@ -355,8 +368,8 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
 #pragma unroll
     for (int j = 0; j < CQ; ++j) {
       if (j >= nq) break;
-      const double* N = P.cqp_N + __ldg(&P.cqp_noff[q0 + j]);
-      const double nn = N[a] * N[b];
+      const double* N = P.cqp_N + d4.z + j * nh;
+      const double nn = __ldg(&N[a]) * __ldg(&N[b]);
 #pragma unroll
       for (int i = 0; i < D2; ++i) blk[i] += nn * Wa[j][i];
     }
@@ -370,7 +383,7 @@ __device__ __forceinline__ void coh_element(const DevProblem& P, int ce, int qi,
 #pragma unroll
     for (int j = 0; j < CQ; ++j) {
       if (j >= nq) break;
-      const double na = P.cqp_N[__ldg(&P.cqp_noff[q0 + j]) + a];
+      const double na = __ldg(&P.cqp_N[d4.z + j * nh + a]);
 #pragma unroll
       for (int i = 0; i < DIM; ++i) t[i] += na * Ta[j][i];
     }

@@ -32,9 +32,10 @@ int shape_consts(pg_ctx* c, const pgd::DevProblem& P, double* out);
 // The rows of one pass; `dependent`: a programmatic dependent launch of the cohesive elements'
 // kernel before it (the rows that do not need its output run beside it).
 template <int DIM, bool CASES>
-void rows(const pgd::DevProblem& P, const pgd::RowParts& parts, bool dependent, cudaStream_t st) {
-  const int blocks = parts.n[0] + parts.n[1] + parts.n[2] + parts.n[3];
+void rows(const pgd::DevProblem& P, pgd::RowParts parts, bool dependent, cudaStream_t st) {
+  const int blocks = parts.total();
   if (blocks == 0) return;
+  parts.spread();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3(pgd::kRowThreads);
@@ -44,8 +45,21 @@ void rows(const pgd::DevProblem& P, const pgd::RowParts& parts, bool dependent, 
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = dependent ? 1 : 0;
-  if (DIM == 2 && P.npe == 4) cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, 36, CASES>, P, parts);
-  else cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, pgd::pattern_period(DIM, DIM + 1), CASES>, P, parts);
+  auto launch = [&](auto per) {
+    constexpr int PER = decltype(per)::value;
+    const bool coh = P.n_coh_el > 0;
+    if constexpr (!CASES) {
+      if (P.flags & PG_JAC) {
+        if (coh) cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, PER, false, true, true>, P, parts);
+        else cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, PER, false, true, false>, P, parts);
+        return;
+      }
+    }
+    if (coh) cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, PER, CASES, false, true>, P, parts);
+    else cudaLaunchKernelEx(&cfg, pgd::k_rows<DIM, PER, CASES, false, false>, P, parts);
+  };
+  if (DIM == 2 && P.npe == 4) launch(pgd::IntC<36>{});
+  else launch(pgd::IntC<pgd::pattern_period(DIM, DIM + 1)>{});
 }
 
 template <int DIM>
@@ -69,9 +83,9 @@ void assembly(pg_ctx* c, const pgd::DevProblem& P) {
   cudaEventRecord(c->ev[0], c->stream);
   cohesive<DIM>(c, P);
   cudaEventRecord(c->ev[1], c->stream);
-  rows<DIM, false>(P, {{0, all.n[1], 0, all.n[3]}}, false, c->stream);
+  rows<DIM, false>(P, {{0, all.n[1], 0, all.n[3]}, false, 0}, false, c->stream);
   cudaEventRecord(c->ev[2], c->stream);
-  rows<DIM, false>(P, {{all.n[0], 0, all.n[2], 0}}, false, c->stream);
+  rows<DIM, false>(P, {{all.n[0], 0, all.n[2], 0}, false, 0}, false, c->stream);
   cudaEventRecord(c->ev[3], c->stream);
   cudaEventRecord(c->ev[4], c->stream);
 }

@@ -143,11 +143,11 @@ __device__ __forceinline__ double* irregular_dst(const DevProblem& P, int node, 
 
 // General node `node` (P.gnd[2 node], P.gnd[2 node + 1]: {first static slot, slots | regular << 16,
 // first CSR value of K_ff (regular), first DOF (regular)}, {first traction, tractions, -, -}) by a
-// group of L lanes, lane g.  JAC: its rows of the matrix; FUNC: its residual entries; CASES: the
+// group of L lanes, lane g.  T: slots (2D) or columns (3D) of a lane in flight.  JAC: its rows of the matrix; FUNC: its residual entries; CASES: the
 // residuals of a multi-strain pass.  COH: a node on a cohesive element (its cohesive blocks and
 // tractions come from the cohesive elements' kernel).  Called by whole groups.
-template <int DIM, bool COH, bool CASES>
-__device__ __forceinline__ void gen_node(const DevProblem& P, int node, bool jac, bool func) {
+template <int DIM, bool COH, bool CASES, bool JAC, int T>
+__device__ __forceinline__ void gen_node(const DevProblem& P, int node, bool func) {
   constexpr int L = GenLanes<DIM>::L, D2 = DIM * DIM, NV = (DIM == 2) ? 3 : 6;
   const int g = threadIdx.x % L;
   const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31) / L * L);
@@ -159,80 +159,122 @@ __device__ __forceinline__ void gen_node(const DevProblem& P, int node, bool jac
   double r[DIM];
 #pragma unroll
   for (int q = 0; q < DIM; ++q) r[q] = 0.0;
+  // T slots (2D) or columns (3D) of a lane at a time: every load that depends on the descriptor
+  // alone is issued before the first one is used
   if constexpr (DIM == 2) {
-    for (int k = g; k < nn; k += L) {
-      const double2 s0 = __ldg(reinterpret_cast<const double2*>(S) + k);
-      const double2 s1 = __ldg(reinterpret_cast<const double2*>(S + pitch) + k);
-      double b[4] = {s0.x, s0.y, s1.x, s1.y};
-      if (func) {
-        double u[2];
-        load_node<2>(P.U, __ldg(&P.stat_node[a.x + k]), u);
-        r[0] = __fma_rn(b[1], u[1], __fma_rn(b[0], u[0], r[0]));
-        r[1] = __fma_rn(b[3], u[1], __fma_rn(b[2], u[0], r[1]));
+    for (int k0 = g; k0 < nn; k0 += T * L) {
+      double b[T][4];
+      int id[T], c0[T], c1[T], cl[T];
+      double u[T][2];
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const int k = k0 + t * L;
+        if (k >= nn) break;
+        const double2 s0 = __ldg(reinterpret_cast<const double2*>(S) + k);
+        const double2 s1 = __ldg(reinterpret_cast<const double2*>(S + pitch) + k);
+        b[t][0] = s0.x; b[t][1] = s0.y; b[t][2] = s1.x; b[t][3] = s1.y;
+        if (func) id[t] = __ldg(&P.stat_node[a.x + k]);
+        if constexpr (COH && JAC) { c0[t] = __ldg(&P.gblk_cl[a.x + k]); c1[t] = __ldg(&P.gblk_cl[a.x + k + 1]); }
       }
-      if (!jac) continue;
-      if constexpr (COH) {
-        const int c0 = __ldg(&P.gblk_cl[a.x + k]), c1 = __ldg(&P.gblk_cl[a.x + k + 1]);
-        if (c1 > c0) dep_wait();
-        for (int j = c0; j < c1; ++j) {
-          const int c = __ldg(&P.gcl[j]);
-          const double sgn = (c & 1) ? -1.0 : 1.0;
-          const double2* B = reinterpret_cast<const double2*>(P.kcoh + (c >> 1));
-          const double2 t0 = B[0], t1 = B[1];
-          b[0] = __fma_rn(sgn, t0.x, b[0]);
-          b[1] = __fma_rn(sgn, t0.y, b[1]);
-          b[2] = __fma_rn(sgn, t1.x, b[2]);
-          b[3] = __fma_rn(sgn, t1.y, b[3]);
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        if (k0 + t * L >= nn) break;
+        if (func) load_node<2>(P.U, id[t], u[t]);
+        if constexpr (COH && JAC) cl[t] = (c1[t] > c0[t]) ? __ldg(&P.gcl[c0[t]]) : 0;
+      }
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const int k = k0 + t * L;
+        if (k >= nn) break;
+        double* e = b[t];
+        if (func) {
+          r[0] = __fma_rn(e[1], u[t][1], __fma_rn(e[0], u[t][0], r[0]));
+          r[1] = __fma_rn(e[3], u[t][1], __fma_rn(e[2], u[t][0], r[1]));
         }
-      }
-      if (regular) {
-        double* v = P.val[0] + a.z + 2 * k;
-        if ((a.z & 1) == 0) {   // (the pitch is even: both rows are aligned, or neither)
-          *reinterpret_cast<double2*>(v) = make_double2(b[0], b[1]);
-          *reinterpret_cast<double2*>(v + pitch) = make_double2(b[2], b[3]);
+        if constexpr (!JAC) continue;
+        if constexpr (COH) {
+          if (c1[t] > c0[t]) dep_wait();
+          int c = cl[t];
+          for (int j = c0[t]; j < c1[t]; ++j) {
+            const int next = (j + 1 < c1[t]) ? __ldg(&P.gcl[j + 1]) : 0;
+            const double sgn = (c & 1) ? -1.0 : 1.0;
+            const double2* B = reinterpret_cast<const double2*>(P.kcoh + (c >> 1));
+            const double2 t0 = B[0], t1 = B[1];
+            e[0] = __fma_rn(sgn, t0.x, e[0]);
+            e[1] = __fma_rn(sgn, t0.y, e[1]);
+            e[2] = __fma_rn(sgn, t1.x, e[2]);
+            e[3] = __fma_rn(sgn, t1.y, e[3]);
+            c = next;
+          }
+        }
+        if (regular) {
+          double* v = P.val[0] + a.z + 2 * k;
+          if ((a.z & 1) == 0) {   // (the pitch is even: both rows are aligned, or neither)
+            *reinterpret_cast<double2*>(v) = make_double2(e[0], e[1]);
+            *reinterpret_cast<double2*>(v + pitch) = make_double2(e[2], e[3]);
+          } else {
+            v[0] = e[0];
+            v[1] = e[1];
+            v[pitch] = e[2];
+            v[pitch + 1] = e[3];
+          }
         } else {
-          v[0] = b[0];
-          v[1] = b[1];
-          v[pitch] = b[2];
-          v[pitch + 1] = b[3];
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int d = 0; d < 2; ++d) *irregular_dst<2>(P, node, q, k, d) = e[q * 2 + d];
         }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int d = 0; d < 2; ++d) *irregular_dst<2>(P, node, q, k, d) = b[q * 2 + d];
       }
     }
   } else {
-    for (int j = g; j < pitch; j += L) {
-      const int k = j / 3, d = j - 3 * k;
-      double b[3];
+    for (int j0 = g; j0 < pitch; j0 += T * L) {
+      double b[T][3], u[T];
+      int id[T], c0[T], c1[T], cl[T];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) b[q] = __ldg(&S[q * pitch + j]);
-      if (func) {
-        const double u = __ldg(&P.U[(size_t)__ldg(&P.stat_node[a.x + k]) * 3 + d]);
+      for (int t = 0; t < T; ++t) {
+        const int j = j0 + t * L;
+        if (j >= pitch) break;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) r[q] = __fma_rn(b[q], u, r[q]);
+        for (int q = 0; q < 3; ++q) b[t][q] = __ldg(&S[q * pitch + j]);
+        if (func) id[t] = __ldg(&P.stat_node[a.x + j / 3]);
+        if constexpr (COH && JAC) { c0[t] = __ldg(&P.gblk_cl[a.x + j / 3]); c1[t] = __ldg(&P.gblk_cl[a.x + j / 3 + 1]); }
       }
-      if (!jac) continue;
-      if constexpr (COH) {
-        const int c0 = __ldg(&P.gblk_cl[a.x + k]), c1 = __ldg(&P.gblk_cl[a.x + k + 1]);
-        if (c1 > c0) dep_wait();
-        for (int i = c0; i < c1; ++i) {
-          const int c = __ldg(&P.gcl[i]);
-          const double sgn = (c & 1) ? -1.0 : 1.0;
-          const double* B = P.kcoh + (c >> 1) + d;
 #pragma unroll
-          for (int q = 0; q < 3; ++q) b[q] = __fma_rn(sgn, B[3 * q], b[q]);
+      for (int t = 0; t < T; ++t) {
+        const int j = j0 + t * L;
+        if (j >= pitch) break;
+        if (func) u[t] = __ldg(&P.U[(size_t)id[t] * 3 + j % 3]);
+        if constexpr (COH && JAC) cl[t] = (c1[t] > c0[t]) ? __ldg(&P.gcl[c0[t]]) : 0;
+      }
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const int j = j0 + t * L;
+        if (j >= pitch) break;
+        if (func) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) r[q] = __fma_rn(b[t][q], u[t], r[q]);
         }
-      }
-      if (regular) {
-        double* v = P.val[0] + a.z + j;
+        if constexpr (!JAC) continue;
+        if constexpr (COH) {
+          if (c1[t] > c0[t]) dep_wait();
+          int c = cl[t];
+          for (int i = c0[t]; i < c1[t]; ++i) {
+            const int next = (i + 1 < c1[t]) ? __ldg(&P.gcl[i + 1]) : 0;
+            const double sgn = (c & 1) ? -1.0 : 1.0;
+            const double* B = P.kcoh + (c >> 1) + j % 3;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) v[q * pitch] = b[q];
-      } else {
+            for (int q = 0; q < 3; ++q) b[t][q] = __fma_rn(sgn, B[3 * q], b[t][q]);
+            c = next;
+          }
+        }
+        if (regular) {
+          double* v = P.val[0] + a.z + j;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) *irregular_dst<3>(P, node, q, k, d) = b[q];
+          for (int q = 0; q < 3; ++q) v[q * pitch] = b[t][q];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) *irregular_dst<3>(P, node, q, j / 3, j % 3) = b[t][q];
+        }
       }
     }
   }
@@ -291,31 +333,71 @@ __global__ void __launch_bounds__(128) k_coh_elements(DevProblem P) {
 
 // A block's work: `part` 0 general nodes without cohesive elements, 1 stencil residuals, 2 general
 // nodes on cohesive elements, 3 CSR chunks; item `b` of the part.  The whole block calls it.
-template <int DIM, int PER, bool CASES>
+template <int DIM, int PER, bool CASES, bool JAC, bool COH>
 __device__ __forceinline__ void row_block(const DevProblem& P, int part, int b) {
   constexpr int GN = kRowThreads / GenLanes<DIM>::L;
-  const bool jac = !CASES && (P.flags & FLAG_JAC) != 0, func = CASES || (P.flags & FLAG_FUNC) != 0;
+  // 3D lanes take several columns at once (22 x 18 x 25 cohesive tet4: 22 us with three, 27 with
+  // one; 64^3 linear 177 with two, 182 with three); 2D ones take one slot, since a second costs
+  // blocks per SM (512 x 512 with 200 fibers: 38 us against 35)
+  constexpr int T = (DIM == 2) ? 1 : (COH ? 3 : 2);
+  const bool func = CASES || (P.flags & FLAG_FUNC) != 0;
   const int t = threadIdx.x;
   if (part == 0) {
     const int node = b * GN + t / GenLanes<DIM>::L;
-    if (node < P.n_gen_plain) gen_node<DIM, false, CASES>(P, node, jac, func);
+    if (node < P.n_gen_plain) gen_node<DIM, false, CASES, JAC, T>(P, node, func);
   } else if (part == 1) {
     const int i = b * kRowThreads + t;
     if (i < P.n_snode) {
       const int4 v = __ldg(&P.snode[i]);
       if (v.x >= 0) node_resid<DIM, CASES>(P, v);   // (-1: padding of a class to whole warps)
     }
-  } else if (part == 2) {
+  } else if (COH && part == 2) {
     const int node = P.n_gen_plain + b * GN + t / GenLanes<DIM>::L;
-    if (node < P.n_slow_dn) gen_node<DIM, true, CASES>(P, node, jac, func);
-  } else {
+    if (node < P.n_slow_dn) gen_node<DIM, true, CASES, JAC, T>(P, node, func);
+  } else if (JAC && part == 3) {
     const int c = b * (kRowThreads / 32) + (t >> 5);
     if (c < P.n_chunk) write_chunk<PER>(P, __ldg(&P.chunk[c]), t & 31);
   }
 }
 
 // Blocks of the parts of an assembly with these outputs.
-struct RowParts { int n[4]; };
+struct RowParts {
+  int n[4];
+  bool mixed;
+  unsigned long long share;   // structured blocks / all blocks, rounded up to a multiple of 2^-32
+  // The part and block of the part that block `b` of the launch takes.  Without cohesive elements the
+  // structured rows' blocks (residuals, then chunks) are spread evenly among the general rows', so
+  // that the stores of the one run beside the long chains of loads of the other from beginning to
+  // end (64^3 tet4, K and R and five residuals: 177 us against 182 part after part).  With them the
+  // parts follow one another, the chunks last: they run when the blocks that wait for the cohesive
+  // elements are done waiting (512 x 512 tri3 with 200 fibers: 34.7 us against 35.6 spread, 37.9
+  // with the waiting blocks last, 37.4 with the chunks first).
+  __host__ __device__ int total() const { return n[0] + n[1] + n[2] + n[3]; }
+  void spread() {
+    const unsigned long long t = (unsigned long long)total(), s = (unsigned long long)(n[1] + n[3]);
+    share = t ? ((s << 32) + t - 1) / t : 0;
+    mixed = n[2] == 0;
+  }
+  __host__ __device__ void pick(int b, int* part, int* item) const {
+    if (!mixed) {
+      *part = 0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (*part == k && b >= n[k]) { b -= n[k]; *part = k + 1; }
+      *item = b;
+      return;
+    }
+    const int before = (int)((unsigned)b * share >> 32);
+    if ((int)(((unsigned)b + 1u) * share >> 32) > before) {
+      *part = before < n[1] ? 1 : 3;
+      *item = before < n[1] ? before : before - n[1];
+    } else {
+      const int g = b - before;
+      *part = g < n[0] ? 0 : 2;
+      *item = g < n[0] ? g : g - n[0];
+    }
+  }
+};
 inline RowParts row_parts(const DevProblem& P, bool jac, bool func, bool cases) {
   const int gn = kRowThreads / ((P.dim == 2) ? GenLanes<2>::L : GenLanes<3>::L);
   auto up = [](int n, int per) { return (n + per - 1) / per; };
@@ -324,23 +406,16 @@ inline RowParts row_parts(const DevProblem& P, bool jac, bool func, bool cases) 
   r.n[1] = (func || cases) ? up(P.n_snode, kRowThreads) : 0;
   r.n[2] = up(P.n_slow_dn - P.n_gen_plain, gn);
   r.n[3] = (jac && !cases) ? up(P.n_chunk, kRowThreads / 32) : 0;
+  r.spread();
   return r;
 }
 
-// The rows of one assembly: the parts' blocks one after another.  The general rows come first (the
-// longest chains of loads; they overlap the chunks' stores), the ones that wait for the cohesive
-// elements after those that do not.
-template <int DIM, int PER, bool CASES>
+// The rows of one assembly (COH: of a mesh with cohesive elements).
+template <int DIM, int PER, bool CASES, bool JAC, bool COH>
 __global__ void __launch_bounds__(kRowThreads) k_rows(DevProblem P, RowParts parts) {
-  int b = blockIdx.x;
-#pragma unroll
-  for (int part = 0; part < 4; ++part) {
-    if (b < parts.n[part]) {
-      row_block<DIM, PER, CASES>(P, part, b);
-      return;
-    }
-    b -= parts.n[part];
-  }
+  int part, item;
+  parts.pick(blockIdx.x, &part, &item);
+  row_block<DIM, PER, CASES, JAC, COH>(P, part, item);
 }
 
 // ---------------------------------------------------------------- set-up

@@ -76,3 +76,16 @@ def test_ply_boundaries_are_general_rows(elem, n):
         t[dofs[:, d]] = 1.0
         assert np.abs(K @ t).max() <= 1e-11 * top
     P.close()
+
+
+@pytest.mark.parametrize("n", [(2, 2), (40, 50), (45, 45), (46, 45), (120, 97)])
+def test_residual_norm_over_block_counts(n):
+    """One block, exactly one and a few more values than a block, several blocks, repeated calls: the
+    norm of the host copy to the rounding of a sum of n squares (1e-13 relative), the same bits twice."""
+    from pigfem_b200 import capi
+    P = capi.Problem(_desc(TRI3, n, [], False, False))
+    U = np.random.default_rng(1).uniform(-1e-3, 1e-3, P.n_nodes * 2)
+    ref = np.linalg.norm(P.assemble(U, 1.0)["P_f"])
+    got = [P.residual_norm() for _ in range(3)]
+    assert abs(got[0] - ref) <= 1e-13 * ref and got[0] == got[1] == got[2]
+    P.close()
