@@ -219,7 +219,7 @@ struct PcgRing {
   bool resident;
   unsigned issued, used;    // chunks fetched / consumed so far
 
-  __device__ __forceinline__ void issue(const PcgArgs& a) {   // one lane
+  __device__ __forceinline__ void issue(const PcgArgs& a, int after) {   // one lane
     const int4 c = __ldg(first + (size_t)(issued % n) * kPcgWarps), e = __ldg(first + (size_t)(issued % n) * kPcgWarps + 1);
     const unsigned st = issued % S::kStages;
     const unsigned full = bar + 8 * st;
@@ -232,7 +232,7 @@ struct PcgRing {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(gb + vb + cb) : "memory");
     auto copy = [&](unsigned to, const void* from, unsigned bytes) {
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
-                   "l"(from), "r"(bytes), "r"(full)
+                   "l"(from), "r"(bytes), "r"(full), "r"(after)
                    : "memory");
     };
     copy(dst, a.grp + c.x, gb);
@@ -249,10 +249,11 @@ struct PcgRing {
     }
     return false;
   }
-  __device__ __forceinline__ void fill(const PcgArgs& a, int lane) {
+  // `after`: a value the copies wait for (they do not use it)
+  __device__ __forceinline__ void fill(const PcgArgs& a, int lane, int after = 0) {
     const unsigned upto = resident ? (unsigned)n : used + S::kStages;
     for (; n > 0 && issued < upto; ++issued)
-      if (lane == 0) issue(a);
+      if (lane == 0) issue(a, after);
   }
   // Waits for every fetch still in flight (before the block returns).
   __device__ __forceinline__ void drain() {
@@ -314,10 +315,18 @@ __device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring
       const double* sv = reinterpret_cast<const double*>(mem + S::kGroups * 16 + S::kColBytes);
       rows(sv + (d.y - (d0.y & ~1)), sc + (d.z - (d0.z & ~3)));
     }
-    __syncwarp();   // the stage is read
     if (!ring.resident) {
+      // The next copy into this stage must not start before every lane's loads from it have
+      // returned (issued is not enough: the copy is not ordered with them), so the warp votes on a
+      // value formed from the sums they went into.
+      int seen = d.w ^ d0.w;
+#pragma unroll
+      for (int r = 0; r < M; ++r)
+#pragma unroll
+        for (int j = 0; j < NS; ++j) seen ^= __double2loint(acc[r][j]);
+      const int vote = __any_sync(0xffffffffu, seen == 0x5a5a5a5a);
       ++ring.used;
-      ring.fill(a, wl);
+      ring.fill(a, wl, vote);
     }
     double qv[NS];
     if constexpr (M == 3) {
