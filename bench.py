@@ -100,7 +100,7 @@ def algorithmic_bytes(P, fp32: bool) -> dict:
 
 
 def fast_kernel_bytes(P, fp32: bool) -> float:
-    """Algorithmic bytes of the dominant kernel (rows whose elements are all uncut): the CSR values
+    """Algorithmic bytes of the structured rows (all their elements uncut): the CSR values
     and residual entries of its rows, plus connectivity/material of the uncut elements and the
     coordinates and U of the standard nodes."""
     s = P.sizes
@@ -124,7 +124,7 @@ def fast_kernel_bytes(P, fp32: bool) -> float:
 
 
 def general_kernel_bytes(P, fp32: bool) -> float:
-    """Algorithmic bytes of the general-row kernel (boundary rows, nodes of cut elements and
+    """Algorithmic bytes of the general rows (boundary rows, nodes of cut elements and
     enrichment nodes): the CSR values and residual entries of its rows, connectivity/material of
     the elements adjacent to them, a 4 B sub-element table index per cut element, and the
     coordinates and U of the nodes their rows couple to."""
@@ -153,15 +153,10 @@ def general_kernel_bytes(P, fp32: bool) -> float:
 
 def launches_per_step(P, three_d: bool = False) -> int:
     """Kernels one step launches (the L2 flush between steps is a torch fill, not counted).  An
-    assembly: k_gen_first (the cohesive elements), the tiles of the structured rows, k_gen_rows
-    (the general rows), each only when it has work.  The 3D step adds the multi-strain residual
-    pass: its cohesive elements, structured rows and general rows."""
-    s = P.sizes
-    fast, slow = len(P.debug("fast_dn")) > 0, len(P.debug("slow_dn")) > 0
-    n = int(s["n_coh_qp"] > 0) + int(fast) + int(slow)
-    if three_d:
-        n += int(s["n_coh_qp"] > 0) + int(fast) + int(slow)
-    return n
+    assembly: k_coh_elements (when there are cohesive elements) and k_rows (all rows).  The 3D
+    step adds the multi-strain residual pass, the same two kernels."""
+    n = int(P.sizes["n_coh_qp"] > 0) + 1
+    return 2 * n if three_d else n
 
 
 class Clocks:
@@ -875,7 +870,8 @@ def main():
     batched = None
     if args.workload == "cohesive_2d_512" and not args.no_batched:
         batched = batched_summary(args, ws, rank)
-    # roofline of the dominant kernel (the fast row kernel), from the live per-kernel events
+    # roofline of the structured rows, which write most of the bytes, from the events around their
+    # own launch (an untimed assembly has all rows in one)
     peak, peak_kind = measured_peak_hbm()
     fk_bytes = fast_kernel_bytes(P, False)
     fk_ms = float(kt64[1])
@@ -886,8 +882,8 @@ def main():
         # the five extra right-hand sides write their residuals (one pass reads the nodes once)
         extra = 5 * 8 * (P.n_free + P.n_const)
         alg["total"] += extra
-    stencil_name = f"k_rows_tile{P.dim}<double,1>"
-    general_name = f"k_gen_rows<{P.dim}>"
+    stencil_name = f"k_rows<{P.dim}>:structured"
+    general_name = f"k_rows<{P.dim}>:general"
     gk_bytes = general_kernel_bytes(P, False)
     gk_ms = float(kt64[2])
     g_achieved = gk_bytes / (gk_ms * 1e-3) / 1e9 if gk_ms > 0 else None
@@ -906,20 +902,20 @@ def main():
                                           "cohesive_qps": P.sizes["n_coh_qp"]}, ws),
             "fp32_mixed": {"value": value32, "unit": UNIT, "ms_per_step": ms32 / args.steps, "speedup_vs_fp64": value32 / value,
                            "kernel_ms": [float(x) for x in kt32]},
-            "kernel_ms": {"cohesive_elements_and_records": float(kt64[0]), "rows_stencil": float(kt64[1]),
+            "kernel_ms": {"cohesive_elements": float(kt64[0]), "rows_stencil": float(kt64[1]),
                           "rows_general": float(kt64[2]), "assembly": float(kt64[3])},
             "algorithmic_bytes_per_step": alg["total"], "algorithmic_bytes_per_element": alg["total"] / ne,
             "algorithmic_gbs": alg["total"] / (ms64 / args.steps * 1e-3) / 1e9,
-            "roofline": {"bound": "hbm", "kernel": f"{stencil_name} " + ("(low-priority stream, concurrent with the cohesive and general-row kernels)" if P.dim == 2 else "(main stream, alone)"),
+            "roofline": {"bound": "hbm", "kernel": f"{stencil_name} (launched by itself)",
                          "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": (achieved / peak) if achieved else None,
-                         "traffic": profiled_traffic(stencil_name), "bytes_per_launch": fk_bytes,
-                         "traffic_note": "ncu dram read+write per launch, cold cache; row writes still in L2 at kernel end are not counted"},
-            # the longest-running kernel (the stencil kernel above moves most of the bytes)
-            "roofline_general": {"bound": "hbm", "kernel": f"{general_name} " + ("(high-priority stream, after the cohesive elements and records, sharing the SMs with the stencil rows)" if P.dim == 2 else "(main stream, after the stencil rows, alone)"),
+                         "traffic": profiled_traffic("k_rows<2,56,0,1,1>") if args.workload == "cohesive_2d_512" else None,
+                         "bytes_per_launch": fk_bytes,
+                         "traffic_note": "ncu dram read+write of the one launch of all rows, cold cache; writes still in L2 at kernel end are not counted"},
+            # the general rows: fewer bytes of output, more per row to read
+            "roofline_general": {"bound": "hbm", "kernel": f"{general_name} (launched by itself)",
                                  "achieved": g_achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-                                 "frac": (g_achieved / peak) if g_achieved else None,
-                                 "traffic": profiled_traffic(general_name), "bytes_per_launch": gk_bytes},
+                                 "frac": (g_achieved / peak) if g_achieved else None, "bytes_per_launch": gk_bytes},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "ms_per_step": e2e_ms / e2e_steps, "steps": e2e_steps,
                     "mode": "PG_KEEP_STATIC: the caller's host K arrays keep the previous call's values; every step "

@@ -172,13 +172,12 @@ int pg_device_outputs(pg_ctx* ctx, double** K_vals4, double** P_f, double** P_p)
 /* Stream the context launches on (a cudaStream_t, 0 = legacy default). */
 int pg_set_stream(pg_ctx* ctx, void* stream);
 
-/* Device timing of the last assembly from CUDA events the context records on its streams:
- * ms[0] cohesive elements and element records, ms[1] stencil rows (2D: side stream, concurrent
- * with ms[0] and ms[2]; 3D: after ms[0]), ms[2] general rows (2D: after ms[0]; 3D: after ms[1]),
- * ms[3] the whole assembly (fork to join).  The event between ms[0] and ms[2] is recorded only
- * while timing is on (pg_set_timing(ctx, 1)): without it the general rows start early, while the
- * kernel before them finishes.  pg_kernel_times returns PG_ERR_STATE when the last assembly ran
- * with timing off. */
+/* Device timing of the last assembly from CUDA events on the context's stream: ms[0] cohesive
+ * elements, ms[1] structured rows, ms[2] general rows, ms[3] the whole assembly.  While timing is
+ * on (pg_set_timing(ctx, 1)) the three run one after another with an event between them; without
+ * it all rows are one launch that starts while the cohesive elements' kernel runs, so ms[3] is
+ * more than an untimed assembly takes.  pg_kernel_times returns PG_ERR_STATE when the last
+ * assembly ran with timing off. */
 int pg_set_timing(pg_ctx* ctx, int on);
 int pg_kernel_times(pg_ctx* ctx, float* ms);
 
@@ -248,13 +247,13 @@ int pg_batch_create(pg_ctx* const* ctxs, int n, pg_batch** out);
 int pg_batch_assemble(pg_batch* b, const double* const* d_U, const double* t_frac, int flags);
 /* Waits for the last pg_batch_assemble; ms (may be NULL) gets its device time. */
 int pg_batch_wait(pg_batch* b, float* ms);
-/* Autotuner: times every candidate launch shape (persistent blocks per SM; the stencil rows run
- * as fixed tiles, the general rows a thread per row block) over `reps` assemblies of this batch
- * and keeps the fastest; best[3] (may be NULL) gets {threads per stencil tile, 1, blocks per SM}.
+/* Autotuner: times every candidate launch shape (persistent blocks per SM) over `reps` assemblies
+ * of this batch and keeps the fastest; best[3] (may be NULL) gets {threads per row block, 1,
+ * blocks per SM}.
  * Contexts must be tri3 or tet4 (PG_ERR_UNSUPPORTED for quad4). */
 int pg_batch_tune(pg_batch* b, const double* const* d_U, int flags, int reps, int* best);
-/* info[8]: contexts, elements, threads per stencil tile, 1, blocks per SM, cohesive-point chunks,
- * stencil chunks, general-row chunks. */
+/* info[8]: contexts, elements, threads per row block, 1, blocks per SM; work items of the cohesive
+ * elements, the structured rows and the general rows. */
 int pg_batch_info(const pg_batch* b, int64_t* info);
 const char* pg_batch_last_error(const pg_batch* b);
 void pg_batch_destroy(pg_batch* b);

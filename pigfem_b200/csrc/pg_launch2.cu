@@ -1,4 +1,4 @@
-// pg_launch2.cu -- the 2D (tri3) kernels and their launches.
+// pg_launch2.cu -- the 2D (tri3, quad4) kernels and their launches.
 #define PG_LAUNCH_IMPL
 #include "pg_launch.cuh"
 

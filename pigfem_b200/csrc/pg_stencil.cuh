@@ -80,7 +80,7 @@ __device__ __forceinline__ void part_iso(const T* d, const T* ga, int q, T* part
   }
 }
 
-// the nonzero entries of an isotropic D (36 entries, row-major) in lei_stress_iso's order
+// the nonzero entries of an isotropic D (36 entries, row-major) in part_iso's order
 template <int DIM, typename T>
 __device__ __forceinline__ void iso_from(const T* D, T* d) {
   constexpr int n = (DIM == 2) ? 5 : 12;
