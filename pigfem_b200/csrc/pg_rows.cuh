@@ -24,7 +24,7 @@
 // One launch for the cohesive elements and one for all rows.  Forming every element once per tile
 // and summing records (the design before) was bound by barriers and shared-memory traffic; a
 // 512 x 512 tri3 RVE with 200 fibers (K and R) took 68 us and takes 35, a 64 x 64 linear one 25 and
-// 6.1 (one launch instead of two with four events), K and six residuals of 64^3 tet4 503 and 182.
+// 6.1 (one launch instead of two with four events), K and six residuals of 64^3 tet4 503 and 177.
 //
 // Every value is a sum in a fixed order: results are bit-reproducible, and a residual-only or a
 // batched assembly forms the bits of the full single one (multiply-adds are explicit, so none are
