@@ -121,9 +121,14 @@ int pg_create_prep_device(const pg_problem_desc* desc, int passes, pg_ctx** out)
 #define PG_PREP_PATTERN 2
 /* Device time in ms of the passes pg_create_prep_device ran (-1 when none ran). */
 int pg_prep_device_ms(const pg_ctx* ctx, double* ms);
-/* Read-only view of a set-up table by name (cut-element quadrature, topology); returns 1 for
- * int32, 2 for float64, 0 for an unknown name.  For tests and tools. */
+/* Read-only view of a set-up table by name (cut-element quadrature, topology; "pcg_shape": the
+ * solver's blocks, chunks, most chunks of a warp, stages of its ring and chunks read without it);
+ * returns 1 for int32, 2 for float64, 0 for an unknown name.  For tests and tools. */
 int pg_debug_array(const pg_ctx* ctx, const char* name, int64_t* n, const void** ptr);
+/* Sets one of the context's test settings, for paths that ordinary meshes do not reach.  For tests.
+ *   "pcg_stage_values"  most matrix values of one chunk of the solver (0: as many as a stage holds);
+ *                       before the first solve */
+int pg_debug_set(pg_ctx* ctx, const char* name, int64_t value);
 void pg_destroy(pg_ctx* ctx);
 const char* pg_last_error(const pg_ctx* ctx);
 int pg_get_sizes(const pg_ctx* ctx, pg_sizes* out);

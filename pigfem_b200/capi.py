@@ -34,7 +34,7 @@ ERRORS = {2: "PG_ERR_INPUT", 3: "PG_ERR_GEOMETRY", 4: "PG_ERR_UNSUPPORTED", 7: "
 
 # Every symbol include/pigfem_b200.h declares.
 EXPORTED = [
-    "pg_create", "pg_create_host", "pg_create_prep_device", "pg_prep_device_ms", "pg_upload", "pg_debug_array", "pg_destroy", "pg_last_error",
+    "pg_create", "pg_create_host", "pg_create_prep_device", "pg_prep_device_ms", "pg_upload", "pg_debug_array", "pg_debug_set", "pg_destroy", "pg_last_error",
     "pg_get_sizes", "pg_device_bytes", "pg_get_pattern", "pg_get_nodes", "pg_assemble", "pg_assemble_device", "pg_residual_strains",
     "pg_device_outputs", "pg_changing_values", "pg_set_stream", "pg_set_isv", "pg_get_isv", "pg_commit_isv",
     "pg_get_damage_zones", "pg_residual_norm", "pg_set_timing", "pg_kernel_times", "pg_set_macro_strain",
@@ -88,6 +88,7 @@ def load_library(path: Optional[str] = None):
         "pg_prep_device_ms": (i32, [vp, ctypes.POINTER(ctypes.c_double)]),
         "pg_upload": (i32, [vp]),
         "pg_debug_array": (i32, [vp, ctypes.c_char_p, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(vp)]),
+        "pg_debug_set": (i32, [vp, ctypes.c_char_p, ctypes.c_int64]),
         "pg_destroy": (None, [vp]),
         "pg_last_error": (ctypes.c_char_p, [vp]),
         "pg_get_sizes": (i32, [vp, ctypes.POINTER(_Sizes)]),
@@ -278,6 +279,9 @@ class Problem:
             return np.zeros(0, np.int32 if kind == 1 else np.float64)
         ct = ctypes.c_int32 if kind == 1 else ctypes.c_double
         return np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ct)), shape=(n.value,)).copy()
+
+    def debug_set(self, name: str, value: int) -> None:
+        self._check(load_library().pg_debug_set(self.h, name.encode(), int(value)))
 
     # ------------------------------------------------------------------ assembly
     def node_major(self, U_dof: np.ndarray) -> np.ndarray:

@@ -753,12 +753,22 @@ int pg_debug_array(const pg_ctx* c, const char* name, int64_t* n, const void** p
       {"fast_dn", c->fast_dn.data(), c->fast_dn.size(), 1}, {"slow_dn", c->slow_dn.data(), c->slow_dn.size(), 1},
       {"dn_node", s.dn_node.data(), s.dn_node.size(), 1}, {"dn_nbr", s.dn_nbr.data(), s.dn_nbr.size(), 1},
       {"dn_nbr_off", s.dn_nbr_off.data(), s.dn_nbr_off.size(), 1}, {"dn_adj", s.dn_adj.data(), s.dn_adj.size(), 1},
-      {"dn_adj_off", s.dn_adj_off.data(), s.dn_adj_off.size(), 1},
+      {"dn_adj_off", s.dn_adj_off.data(), s.dn_adj_off.size(), 1}, {"pcg_shape", c->pcg.shape, 5, 1},
   };
   for (auto& t : tab)
     if (std::strcmp(t.k, name) == 0) { *n = (int64_t)t.n; *ptr = t.p; return t.kind; }
   *n = 0; *ptr = nullptr;
   return 0;
+}
+
+int pg_debug_set(pg_ctx* c, const char* name, int64_t value) {
+  if (!c || !name) return PG_ERR_INPUT;
+  if (std::strcmp(name, "pcg_stage_values") == 0) {
+    if (value < 0 || value > 0xffff || c->pcg.grp) return set_err(c, PG_ERR_INPUT, "pcg_stage_values: before the first solve, at most 65535");
+    c->pcg.stage_values = (int)value;
+    return 0;
+  }
+  return set_err(c, PG_ERR_INPUT, "pg_debug_set: unknown name");
 }
 
 int pg_set_timing(pg_ctx* c, int on) {

@@ -28,6 +28,8 @@ struct PcgWork {
   int* hflag = nullptr;                         // pinned host copies of flag (two launches in flight)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev = nullptr, evc[2] = {nullptr, nullptr};
+  int stage_values = 0;                         // most values of a chunk (pg_debug_set; 0: a stage's)
+  int shape[5] = {0, 0, 0, 0, 0};               // blocks, chunks, most chunks of a warp, its ring's stages, chunks read directly
 };
 
 struct pg_ctx {

@@ -219,7 +219,7 @@ struct PcgRing {
   bool resident;
   unsigned issued, used;    // chunks fetched / consumed so far
 
-  __device__ __forceinline__ void issue(const PcgArgs& a, int after) {   // one lane
+  __device__ __forceinline__ void issue(const PcgArgs& a) {   // one lane
     const int4 c = __ldg(first + (size_t)(issued % n) * kPcgWarps), e = __ldg(first + (size_t)(issued % n) * kPcgWarps + 1);
     const unsigned st = issued % S::kStages;
     const unsigned full = bar + 8 * st;
@@ -232,7 +232,7 @@ struct PcgRing {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(gb + vb + cb) : "memory");
     auto copy = [&](unsigned to, const void* from, unsigned bytes) {
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
-                   "l"(from), "r"(bytes), "r"(full), "r"(after)
+                   "l"(from), "r"(bytes), "r"(full)
                    : "memory");
     };
     copy(dst, a.grp + c.x, gb);
@@ -249,11 +249,22 @@ struct PcgRing {
     }
     return false;
   }
-  // `after`: a value the copies wait for (they do not use it)
-  __device__ __forceinline__ void fill(const PcgArgs& a, int lane, int after = 0) {
+  __device__ __forceinline__ void fill(const PcgArgs& a, int lane) {
     const unsigned upto = resident ? (unsigned)n : used + S::kStages;
     for (; n > 0 && issued < upto; ++issued)
-      if (lane == 0) issue(a, after);
+      if (lane == 0) issue(a);
+  }
+  // The stage in use is done with: fetches the chunk that follows into it.  The copy's writes come
+  // after every lane's loads from the stage: each lane's proxy fence orders its own loads before
+  // copies, and __syncwarp orders the lanes before the one that issues the copy.  (__syncwarp alone
+  // does not: it says nothing about the async proxy, and a copy was seen to start with loads issued
+  // but not yet returned.  An mbarrier that all 32 lanes arrive on orders them too, but its arrivals
+  // go one by one: 40^3 tet4 with six right-hand sides 114 us per iteration.)
+  __device__ __forceinline__ void refill(const PcgArgs& a, int lane) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    ++used;
+    fill(a, lane);
   }
   // Waits for every fetch still in flight (before the block returns).
   __device__ __forceinline__ void drain() {
@@ -315,19 +326,6 @@ __device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring
       const double* sv = reinterpret_cast<const double*>(mem + S::kGroups * 16 + S::kColBytes);
       rows(sv + (d.y - (d0.y & ~1)), sc + (d.z - (d0.z & ~3)));
     }
-    if (!ring.resident) {
-      // The next copy into this stage must not start before every lane's loads from it have
-      // returned (issued is not enough: the copy is not ordered with them), so the warp votes on a
-      // value formed from the sums they went into.
-      int seen = d.w ^ d0.w;
-#pragma unroll
-      for (int r = 0; r < M; ++r)
-#pragma unroll
-        for (int j = 0; j < NS; ++j) seen ^= __double2loint(acc[r][j]);
-      const int vote = __any_sync(0xffffffffu, seen == 0x5a5a5a5a);
-      ++ring.used;
-      ring.fill(a, wl, vote);
-    }
     double qv[NS];
     if constexpr (M == 3) {
       const bool hi = (lane & 4) != 0, odd = (lane & 2) != 0;
@@ -349,6 +347,7 @@ __device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring
         qv[j] = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 1));
       }
     }
+    if (!ring.resident) ring.refill(a, wl);   // (the sums above have used every value of the stage)
     if (writer) {
       store_ns<NS>(a.q, d.x + mine, qv);
 #pragma unroll
@@ -578,8 +577,9 @@ PcgKernels pcg_kernels(int dim) {
 
 // Row groups and chunks of K_ff: the consecutive rows of one DOF node share one column list.
 template <int M>
-void pcg_groups(const pg::Setup& s, std::vector<int4>& grp, std::vector<int>& gci, std::vector<int4>& chunk) {
+void pcg_groups(const pg::Setup& s, int stage_values, std::vector<int4>& grp, std::vector<int>& gci, std::vector<int4>& chunk) {
   using S = PcgShape<M>;
+  const int val_bytes = stage_values > 0 ? std::min(stage_values * 8, S::kValBytes) : S::kValBytes;
   const int n = s.n_free;
   const std::vector<int>& rp = s.rp[0];
   std::vector<int> owner(n, -1);
@@ -607,7 +607,7 @@ void pcg_groups(const pg::Setup& s, std::vector<int4>& grp, std::vector<int>& gc
     const int v1 = rp[r + m], c1 = (int)gci.size() + len;
     // (with the 16-byte boundaries the copies start and end on)
     auto fits = [&](int v0, int c0) {
-      return (((v1 + 1) & ~1) - (v0 & ~1)) * 8 <= S::kValBytes && (((c1 + 3) & ~3) - (c0 & ~3)) * 4 <= S::kColBytes;
+      return (((v1 + 1) & ~1) - (v0 & ~1)) * 8 <= val_bytes && (((c1 + 3) & ~3) - (c0 & ~3)) * 4 <= S::kColBytes;
     };
     if (open == S::kGroups || (open && !fits(chunk.back().z, chunk.back().w))) close(false);
     if (!open) chunk.push_back(make_int4((int)grp.size(), 0, rp[r], (int)gci.size()));
@@ -637,8 +637,8 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
   if (!w.grp) {
     std::vector<int4> grp, chunk;
     std::vector<int> gci;
-    if (dim == 3) pcg_groups<3>(s, grp, gci, chunk);
-    else pcg_groups<2>(s, grp, gci, chunk);
+    if (dim == 3) pcg_groups<3>(s, w.stage_values, grp, gci, chunk);
+    else pcg_groups<2>(s, w.stage_values, grp, gci, chunk);
     for (const int4& d : grp)
       if (grp_len(d.w) >= 0x1000000 - 1) return pg_set_err(c, PG_ERR_UNSUPPORTED, "a row of K_ff with 2^24 entries");
     const int ng = (int)grp.size(), nch = (int)chunk.size() - 1;
@@ -658,6 +658,12 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
       while (b < w.nb && acc >= total * b / w.nb) part[b++] = k + 1;
     }
     w.ng = ng;
+    w.shape[0] = w.nb;
+    w.shape[1] = nch;
+    w.shape[2] = w.shape[4] = 0;
+    for (int b = 0; b < w.nb; ++b) w.shape[2] = std::max(w.shape[2], (part[b + 1] - part[b] + kPcgWarps - 1) / kPcgWarps);
+    w.shape[3] = dim == 3 ? PcgShape<3>::kStages : PcgShape<2>::kStages;
+    for (int k = 0; k < nch; ++k) w.shape[4] += (chunk[k].y & 256) != 0;
     gci.resize((gci.size() + 7) & ~(size_t)3);   // the last chunk's copy ends on a 16-byte boundary
     rc |= pg_dalloc(c, grp.size(), &w.grp) | pg_dalloc(c, gci.size(), &w.gci) | pg_dalloc(c, chunk.size(), &w.chunk) |
           pg_dalloc(c, part.size(), &w.part_of) | pg_dalloc(c, (size_t)n, &w.dinv) | pg_dalloc(c, 1, &w.bar);
