@@ -127,7 +127,9 @@ int pg_prep_device_ms(const pg_ctx* ctx, double* ms);
 int pg_debug_array(const pg_ctx* ctx, const char* name, int64_t* n, const void** ptr);
 /* Sets one of the context's test settings, for paths that ordinary meshes do not reach.  For tests.
  *   "pcg_stage_values"  most matrix values of one chunk of the solver (0: as many as a stage holds);
- *                       before the first solve */
+ *                       before the first solve
+ *   "fail_alloc"        which allocation of the context's working memory fails, counted from the
+ *                       next one (0: none) */
 int pg_debug_set(pg_ctx* ctx, const char* name, int64_t value);
 void pg_destroy(pg_ctx* ctx);
 const char* pg_last_error(const pg_ctx* ctx);

@@ -768,6 +768,10 @@ int pg_debug_set(pg_ctx* c, const char* name, int64_t value) {
     c->pcg.stage_values = (int)value;
     return 0;
   }
+  if (std::strcmp(name, "fail_alloc") == 0) {
+    c->fail_alloc = (int)value;
+    return 0;
+  }
   return set_err(c, PG_ERR_INPUT, "pg_debug_set: unknown name");
 }
 

@@ -52,6 +52,7 @@ struct pg_ctx {
   int n_coh_qp = 0;
   bool assembled = false;
   bool timed_last = false;   // the last assembly recorded every timing event (pg_kernel_times)
+  int fail_alloc = 0;        // the allocation from here on that fails (pg_debug_set; 0: none)
   double prep_ms = -1.0;   // device time of the preprocessing passes (pg_create_prep_device), -1 if none ran
   // PG_KEEP_STATIC: the first CSR value of each block from which a later assembly can change
   // values (the rows of DOFs of nodes on cohesive elements; nnz when no value can change), and
@@ -123,7 +124,11 @@ int pg_dalloc(pg_ctx* c, size_t n, T** out) {
   if (n == 0) n = 1;
   if (int rc = pg_alloc_stream(c)) return rc;
   void* p = nullptr;
-  if (cudaMallocAsync(&p, n * sizeof(T), c->up) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "device allocation failed");
+  const bool fail = c->fail_alloc > 0 && --c->fail_alloc == 0;
+  if (fail || cudaMallocAsync(&p, n * sizeof(T), c->up) != cudaSuccess) {
+    cudaGetLastError();   // (reported here; a later call's check is for its own launches)
+    return pg_set_err(c, PG_ERR_DEVICE, "device allocation failed");
+  }
   pg_track_alloc(c, p, n * sizeof(T));
   cudaMemsetAsync(p, 0, n * sizeof(T), c->up);
   *out = (T*)p;

@@ -625,13 +625,25 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
   PcgWork& w = c->pcg;
   const pg::Setup& s = c->s;
   const int n = s.n_free, dim = s.dim;
+  // (every part is recorded once it is whole: a call after a failed one builds it again)
   if (!w.stream) {
-    if (cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&w.ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&w.evc[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&w.evc[1], cudaEventDisableTiming) != cudaSuccess)
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    int* h = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t& e : ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaMallocHost(&h, sizeof(int) * 64) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e);
+      if (st) cudaStreamDestroy(st);
       return pg_set_err(c, PG_ERR_DEVICE, "solver stream creation failed");
-    if (cudaMallocHost(&w.hflag, sizeof(int) * 64) != cudaSuccess) return pg_set_err(c, PG_ERR_DEVICE, "pinned flag allocation failed");
+    }
+    w.stream = st;
+    w.ev = ev[0];
+    w.evc[0] = ev[1];
+    w.evc[1] = ev[2];
+    w.hflag = h;
   }
   int rc = 0;
   if (!w.grp) {
@@ -657,6 +669,31 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
       acc += weight(k);
       while (b < w.nb && acc >= total * b / w.nb) part[b++] = k + 1;
     }
+    gci.resize((gci.size() + 7) & ~(size_t)3);   // the last chunk's copy ends on a 16-byte boundary
+    int4 *d_grp = nullptr, *d_chunk = nullptr;
+    int *d_gci = nullptr, *d_part = nullptr;
+    double* d_dinv = nullptr;
+    unsigned* d_bar = nullptr;
+    rc = pg_dalloc(c, grp.size(), &d_grp) | pg_dalloc(c, gci.size(), &d_gci) | pg_dalloc(c, chunk.size(), &d_chunk) |
+         pg_dalloc(c, part.size(), &d_part) | pg_dalloc(c, (size_t)n, &d_dinv) | pg_dalloc(c, 1, &d_bar);
+    auto copy = [&](void* d, const void* h, size_t bytes) {
+      return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->up) != cudaSuccess;
+    };
+    if (!rc && (copy(d_grp, grp.data(), grp.size() * sizeof(int4)) || copy(d_gci, gci.data(), gci.size() * sizeof(int)) ||
+                copy(d_chunk, chunk.data(), chunk.size() * sizeof(int4)) || copy(d_part, part.data(), part.size() * sizeof(int)) ||
+                pg_alloc_sync(c)))
+      rc = pg_set_err(c, PG_ERR_DEVICE, "solver tables: copy failed");
+    if (rc) {
+      for (void* p : {(void*)d_grp, (void*)d_gci, (void*)d_chunk, (void*)d_part, (void*)d_dinv, (void*)d_bar})
+        if (p) pg_untrack_free(c, p);
+      return PG_ERR_DEVICE;
+    }
+    w.grp = d_grp;
+    w.gci = d_gci;
+    w.chunk = d_chunk;
+    w.part_of = d_part;
+    w.dinv = d_dinv;
+    w.bar = d_bar;
     w.ng = ng;
     w.shape[0] = w.nb;
     w.shape[1] = nch;
@@ -664,30 +701,27 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
     for (int b = 0; b < w.nb; ++b) w.shape[2] = std::max(w.shape[2], (part[b + 1] - part[b] + kPcgWarps - 1) / kPcgWarps);
     w.shape[3] = dim == 3 ? PcgShape<3>::kStages : PcgShape<2>::kStages;
     for (int k = 0; k < nch; ++k) w.shape[4] += (chunk[k].y & 256) != 0;
-    gci.resize((gci.size() + 7) & ~(size_t)3);   // the last chunk's copy ends on a 16-byte boundary
-    rc |= pg_dalloc(c, grp.size(), &w.grp) | pg_dalloc(c, gci.size(), &w.gci) | pg_dalloc(c, chunk.size(), &w.chunk) |
-          pg_dalloc(c, part.size(), &w.part_of) | pg_dalloc(c, (size_t)n, &w.dinv) | pg_dalloc(c, 1, &w.bar);
-    if (rc) return PG_ERR_DEVICE;
-    if (cudaMemcpyAsync(w.grp, grp.data(), grp.size() * sizeof(int4), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
-        cudaMemcpyAsync(w.gci, gci.data(), gci.size() * sizeof(int), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
-        cudaMemcpyAsync(w.chunk, chunk.data(), chunk.size() * sizeof(int4), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
-        cudaMemcpyAsync(w.part_of, part.data(), part.size() * sizeof(int), cudaMemcpyHostToDevice, c->up) != cudaSuccess ||
-        pg_alloc_sync(c))
-      return pg_set_err(c, PG_ERR_DEVICE, "solver tables: copy failed");
   }
   if (w.cap_rhs < nrhs) {
     // (a solve returns with its work done, so the smaller buffers are idle)
-    for (double* p : {w.r, w.p, w.q, w.xi, w.part, w.sc}) if (p) pg_untrack_free(c, p);
-    if (w.flag) pg_untrack_free(c, w.flag);
-    w.r = w.p = w.q = w.xi = w.part = w.sc = nullptr;
-    w.flag = nullptr;
-    w.cap_rhs = 0;
+    auto drop = [&]() {
+      for (double** p : {&w.r, &w.p, &w.q, &w.xi, &w.part, &w.sc}) {
+        if (*p) pg_untrack_free(c, *p);
+        *p = nullptr;
+      }
+      if (w.flag) pg_untrack_free(c, w.flag);
+      w.flag = nullptr;
+      w.cap_rhs = 0;
+    };
+    drop();
     rc |= pg_dalloc(c, (size_t)n * nrhs, &w.r) | pg_dalloc(c, (size_t)n * nrhs, &w.p) | pg_dalloc(c, (size_t)n * nrhs, &w.q) |
           pg_dalloc(c, (size_t)n * nrhs, &w.xi) | pg_dalloc(c, (size_t)3 * nrhs * w.nb, &w.part) | pg_dalloc(c, (size_t)S_NSC * nrhs, &w.sc) |
           pg_dalloc(c, (size_t)2 * nrhs + F_N, &w.flag);
-    if (rc) return PG_ERR_DEVICE;
+    if (rc || pg_alloc_sync(c)) {
+      drop();
+      return PG_ERR_DEVICE;
+    }
     w.cap_rhs = nrhs;
-    return pg_alloc_sync(c);
   }
   return 0;
 }
