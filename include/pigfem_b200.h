@@ -128,6 +128,9 @@ int pg_debug_array(const pg_ctx* ctx, const char* name, int64_t* n, const void**
 /* Sets one of the context's test settings, for paths that ordinary meshes do not reach.  For tests.
  *   "pcg_stage_values"  most matrix values of one chunk of the solver (0: as many as a stage holds);
  *                       before the first solve
+ *   "pcg_wait_ms"       how long a wait inside the solver's kernel lasts (0: the default, seconds)
+ *   "pcg_missing"       arrivals that the grid barriers of a solve's later launches wait for although
+ *                       none will come (0: none): the solve runs into that limit, PG_ERR_DEVICE
  *   "fail_alloc"        which allocation of the context's working memory fails, counted from the
  *                       next one (0: none) */
 int pg_debug_set(pg_ctx* ctx, const char* name, int64_t value);

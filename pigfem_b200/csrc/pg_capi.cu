@@ -768,6 +768,11 @@ int pg_debug_set(pg_ctx* c, const char* name, int64_t value) {
     c->pcg.stage_values = (int)value;
     return 0;
   }
+  if (std::strcmp(name, "pcg_wait_ms") == 0 || std::strcmp(name, "pcg_missing") == 0) {
+    if (value < 0 || value > 10000) return set_err(c, PG_ERR_INPUT, "pg_debug_set: value out of range");
+    (name[4] == 'w' ? c->pcg.wait_ms : c->pcg.missing) = (int)value;
+    return 0;
+  }
   if (std::strcmp(name, "fail_alloc") == 0) {
     c->fail_alloc = (int)value;
     return 0;

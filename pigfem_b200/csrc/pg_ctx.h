@@ -29,6 +29,7 @@ struct PcgWork {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev = nullptr, evc[2] = {nullptr, nullptr};
   int stage_values = 0;                         // most values of a chunk (pg_debug_set; 0: a stage's)
+  int wait_ms = 0, missing = 0;                 // limit of the kernel's waits (0: the default), arrivals its barriers wait for in vain
   int shape[5] = {0, 0, 0, 0, 0};               // blocks, chunks, most chunks of a warp, its ring's stages, chunks read directly
 };
 

@@ -25,7 +25,9 @@ constexpr int kPcgThreads = 512;      // one block per SM: 128 registers a threa
 constexpr int kPcgWarps = kPcgThreads / 32;
 constexpr int kMaxRhs = 6;            // right-hand sides of one pass (the unit strains of a 3D homogenization)
 constexpr int kRound = 16;            // the host's iteration limit is a multiple of this
-constexpr unsigned kSpinLimit = 1u << 23;   // polls of one grid barrier (seconds) before it gives up
+// How long a wait inside the kernel lasts before it gives up: other blocks and fetches arrive within
+// milliseconds, on a GPU that several processes share within its time slices.
+constexpr unsigned long long kWaitNs = 4000000000ull;
 // scalar slots per right-hand side in PcgWork::sc
 enum { S_RZ = 0, S_BB, S_RELRES, S_NSC };
 // word slots after the 2 x NS per-right-hand-side words of PcgWork::flag
@@ -71,7 +73,14 @@ struct PcgArgs {
   double* sc;             // [NS][S_NSC]
   int* flag;              // [0, NS) done, [NS, 2 NS) iterations, then F_*
   unsigned* bar;          // arrivals at the grid barriers of this solve
+  unsigned long long wait_ns;   // limit of a wait
 };
+
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 
 // NS adjacent doubles (16-byte pairs when NS is even).  Plain loads: p and q change during the
 // kernel, and the grid barrier's acquire makes the other blocks' values visible.
@@ -174,19 +183,25 @@ __device__ __forceinline__ void block_sums(double* v, double (*red)[3 * kMaxRhs]
 }
 
 // All blocks of the (cooperative) launch meet: the arrivals of a solve are counted in one word
-// that only grows, `target` is its value once every block has arrived.  Bounded: false once the
-// limit is reached (the caller returns and the host reports it).
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* stuck) {
+// that only grows, `target` is its value once every block has arrived.  Bounded in time: false once
+// the limit is reached (the caller returns and the host reports it).
+__device__ __forceinline__ bool grid_barrier(const PcgArgs& a, unsigned target, int* stuck) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    unsigned got, spins = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(bar) : "memory");
-    } while ((int)(got - target) < 0 && ++spins < kSpinLimit);
-    ok = (int)(got - target) >= 0;
-    if (!ok) atomicOr(stuck, 1);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    auto arrived = [&]() {
+      unsigned got;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(a.bar) : "memory");
+      return (int)(got - target) >= 0;
+    };
+    bool in = arrived();
+    if (!in) {
+      const unsigned long long t0 = now_ns();
+      while (!(in = arrived()) && now_ns() - t0 < a.wait_ns) {}
+    }
+    ok = in;
+    if (!in) atomicOr(stuck, 1);
   }
   __syncthreads();
   return ok != 0;
@@ -239,15 +254,19 @@ struct PcgRing {
     if (cb) copy(dst + S::kGroups * 16, a.gci + c0, cb);
     if (vb) copy(dst + S::kGroups * 16 + S::kColBytes, a.val + v0, vb);
   }
-  // Waits (bounded) for stage st's fetch number `turn`; the whole warp calls it and agrees.
-  __device__ __forceinline__ bool wait(unsigned st, unsigned turn) const {
-    for (unsigned k = 0; k < kSpinLimit; ++k) {
+  // Waits (bounded in time) for stage st's fetch number `turn`; the whole warp calls it and agrees.
+  __device__ __forceinline__ bool wait(const PcgArgs& a, unsigned st, unsigned turn) const {
+    auto arrived = [&]() {
       unsigned ok;
       asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                    : "=r"(ok) : "r"(bar + 8 * st), "r"(turn & 1u) : "memory");
-      if (__all_sync(0xffffffffu, ok)) return true;
-    }
-    return false;
+      return __all_sync(0xffffffffu, ok) != 0;
+    };
+    if (arrived()) return true;
+    const unsigned long long t0 = now_ns();
+    while (!arrived())
+      if (__any_sync(0xffffffffu, now_ns() - t0 >= a.wait_ns)) return false;
+    return true;
   }
   __device__ __forceinline__ void fill(const PcgArgs& a, int lane) {
     const unsigned upto = resident ? (unsigned)n : used + S::kStages;
@@ -267,9 +286,9 @@ struct PcgRing {
     fill(a, lane);
   }
   // Waits for every fetch still in flight (before the block returns).
-  __device__ __forceinline__ void drain() {
-    if (resident) { for (unsigned k = 0; used == 0 && k < issued; ++k) wait(k, 0); return; }
-    for (; used < issued; ++used) wait(used % S::kStages, used / S::kStages);
+  __device__ __forceinline__ void drain(const PcgArgs& a) {
+    if (resident) { for (unsigned k = 0; used == 0 && k < issued; ++k) wait(a, k, 0); return; }
+    for (; used < issued; ++used) wait(a, used % S::kStages, used / S::kStages);
   }
 };
 
@@ -287,7 +306,7 @@ __device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring
   for (int j = 0; j < NS; ++j) pq[j] = 0.0;
   for (int i = 0; i < ring.n; ++i) {
     const unsigned st = ring.resident ? (unsigned)i : ring.used % S::kStages;
-    if (!ring.wait(st, ring.resident ? 0u : ring.used / S::kStages)) return false;
+    if (!ring.wait(a, st, ring.resident ? 0u : ring.used / S::kStages)) return false;
     const unsigned char* mem = ring.mem + st * pcg_stage_bytes<M>();
     const int4* sg = reinterpret_cast<const int4*>(mem);
     const int4 d0 = sg[0];
@@ -414,7 +433,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
   // a barrier or a fetch that gave up: the block waits for its own copies and returns
   auto give_up = [&]() {
     if (!fine) atomicOr(stuck, 1);
-    ring.drain();
+    ring.drain(a);
   };
   if (first) {
     fine = block_product<NS, M>(a, ring, sum);
@@ -436,7 +455,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
       store_ns<NS>(a.r, i, rv);
     }
     block_sums<3 * NS>(sum, red, a.part, a.nb);
-    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    if (!grid_barrier(a, target += a.nb, stuck)) { give_up(); return; }
     total_sums<3 * NS>(a.part, a.nb, tot);
     if (t == 0) {
       active = 0;
@@ -458,7 +477,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
       for (int j = 0; j < NS; ++j) rv[j] = __dmul_rn(di, rv[j]);
       store_ns<NS>(a.p, i, rv);
     }
-    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    if (!grid_barrier(a, target += a.nb, stuck)) { give_up(); return; }
   } else {
     if (t < NS) {
       rz[t] = a.sc[t * S_NSC + S_RZ];
@@ -474,7 +493,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
     fine = block_product<NS, M>(a, ring, sum);
     if (!__syncthreads_and(fine)) { give_up(); return; }
     block_sums<NS>(sum, red, a.part, a.nb);
-    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    if (!grid_barrier(a, target += a.nb, stuck)) { give_up(); return; }
     total_sums<NS>(a.part, a.nb, tot);
     if (t < NS) step[t] = rz[t] / tot[t];
     __syncthreads();
@@ -503,7 +522,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
     }
     // (the second set of partials: a block may still be reading the first)
     block_sums<2 * NS>(sum, red, a.part + NS * a.nb, a.nb);
-    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    if (!grid_barrier(a, target += a.nb, stuck)) { give_up(); return; }
     total_sums<2 * NS>(a.part + NS * a.nb, a.nb, tot);
     if (t < NS) {
       coef[t] = tot[t] / rz[t];
@@ -547,9 +566,9 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
       }
       active = n_act;
     }
-    if (!grid_barrier(a.bar, target += a.nb, stuck)) { give_up(); return; }
+    if (!grid_barrier(a, target += a.nb, stuck)) { give_up(); return; }
   }
-  ring.drain();
+  ring.drain(a);
   __syncthreads();
   if (blockIdx.x == 0) {
     if (t < NS) {
@@ -732,7 +751,7 @@ int pcg_pass(pg_ctx* c, const double* d_b, double* d_x, int nrhs, double rtol, i
   PcgWork& w = c->pcg;
   const int n = c->s.n_free;
   PcgArgs a{w.grp, w.gci, w.chunk, w.part_of, c->P.val[0], n, w.ng, w.nb, rtol, d_b, d_x,
-            w.dinv, w.r, w.p, w.q, w.xi, w.part, w.sc, w.flag, w.bar};
+            w.dinv, w.r, w.p, w.q, w.xi, w.part, w.sc, w.flag, w.bar, w.wait_ms > 0 ? w.wait_ms * 1000000ull : kWaitNs};
   PcgKernels k;
   switch (nrhs) {
     case 1: k = pcg_kernels<1>(c->s.dim); break;
@@ -765,6 +784,7 @@ int pcg_pass(pg_ctx* c, const double* d_b, double* d_x, int nrhs, double rtol, i
         break;
       }
       arrived += (unsigned)(w.nb * (3 * (it1 - it0) + (first ? 2 : 0)));
+      if (first) arrived += (unsigned)w.missing;   // (pg_debug_set: none in earnest)
       it = it1;
     }
     cudaMemcpyAsync(w.hflag + 32 * (l & 1), w.flag, sizeof(int) * n_flag, cudaMemcpyDeviceToHost, w.stream);
@@ -787,7 +807,7 @@ int pcg_pass(pg_ctx* c, const double* d_b, double* d_x, int nrhs, double rtol, i
   if (rc) return rc;
   const int* f = w.hflag;
   if (f[2 * nrhs + F_BAD]) return pg_set_err(c, PG_ERR_NONFINITE, "K_ff has a non-positive or non-finite diagonal entry");
-  if (f[2 * nrhs + F_STUCK]) return pg_set_err(c, PG_ERR_DEVICE, "a grid barrier of the solver ran out");
+  if (f[2 * nrhs + F_STUCK]) return pg_set_err(c, PG_ERR_DEVICE, "a wait of the solver ran out");
   for (int s = 0; s < nrhs; ++s) {
     const double rr = sc[(size_t)s * S_NSC + S_RELRES];
     if (iters) iters[s] = f[nrhs + s];
