@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128) k_pcg_prepare(PcgArgs a) {
 template <int NS>
 __global__ void __launch_bounds__(128) k_pcg_finish(PcgArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+  if (i >= a.n || a.flag[2 * NS + F_STUCK]) return;   // (out of step: the caller's x stays)
   double xv[NS];
   load_ns<NS>(a.xi, i, xv);
 #pragma unroll
@@ -198,7 +198,9 @@ __device__ __forceinline__ bool grid_barrier(const PcgArgs& a, unsigned target, 
     bool in = arrived();
     if (!in) {
       const unsigned long long t0 = now_ns();
-      while (!(in = arrived()) && now_ns() - t0 < a.wait_ns) {}
+      // (a block that gave up arrives nowhere any more: the others need not wait out their limit)
+      for (unsigned k = 1; !(in = arrived()); ++k)
+        if (k % 64 == 0 && (now_ns() - t0 >= a.wait_ns || *(volatile int*)stuck != 0)) break;
     }
     ok = in;
     if (!in) atomicOr(stuck, 1);
@@ -394,9 +396,13 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first
   __shared__ double red[kPcgWarps][3 * kMaxRhs];
   __shared__ double tot[3 * kMaxRhs];
   __shared__ double rz[kMaxRhs], bb[kMaxRhs], relres[kMaxRhs], step[kMaxRhs], coef[kMaxRhs];
-  __shared__ int done[kMaxRhs], iters[kMaxRhs], active;
+  __shared__ int done[kMaxRhs], iters[kMaxRhs], active, leave;
   const int t = threadIdx.x;
-  if (a.flag[2 * NS + F_BAD]) return;   // set before this launch
+  // Set before this launch (F_STUCK also by a block of this one that gave up already): the launch
+  // queued behind one that gave up would wait for arrivals that never came.
+  if (t == 0) leave = a.flag[2 * NS + F_BAD] | *(volatile int*)&a.flag[2 * NS + F_STUCK];
+  __syncthreads();
+  if (leave != 0) return;   // (read once: the whole block leaves or stays)
   extern __shared__ __align__(16) unsigned char stages[];
   const int c0 = __ldg(&a.part_of[blockIdx.x]), c1 = __ldg(&a.part_of[blockIdx.x + 1]);
   int r0 = 0, r1 = 0;
