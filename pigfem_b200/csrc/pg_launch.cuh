@@ -123,10 +123,10 @@ int shape_consts(pg_ctx* c, const pgd::DevProblem& P, double* out) {
   double* dout = nullptr;
   if (cudaMallocAsync(&dout, bytes, c->up) != cudaSuccess) return 1;
   if constexpr (DIM == 2) {
-    if (P.npe == 4) pgd::k_shape_consts<2, 4><<<1, 32, 0, c->up>>>(P, d.lo[0], d.lo[1], 0.0, h[0], h[1], 0.0, dout);
-    else pgd::k_shape_consts<2, 3><<<1, 32, 0, c->up>>>(P, d.lo[0], d.lo[1], 0.0, h[0], h[1], 0.0, dout);
+    if (P.npe == 4) pgd::k_shape_consts<2, 4><<<1, 32, 0, c->up>>>(P, h[0], h[1], 0.0, dout);
+    else pgd::k_shape_consts<2, 3><<<1, 32, 0, c->up>>>(P, h[0], h[1], 0.0, dout);
   } else {
-    pgd::k_shape_consts<3, 4><<<1, 32, 0, c->up>>>(P, d.lo[0], d.lo[1], d.lo[2], h[0], h[1], h[2], dout);
+    pgd::k_shape_consts<3, 4><<<1, 32, 0, c->up>>>(P, h[0], h[1], h[2], dout);
   }
   cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, c->up);
   cudaFreeAsync(dout, c->up);

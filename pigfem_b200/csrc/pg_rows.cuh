@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(DevProblem P, RowParts par
 }
 
 // ---------------------------------------------------------------- set-up
-// Shape constants of a mesh from the corners of its first cells, one thread: per shape and material
+// Shape constants of a mesh from the corners of a cell at the origin, one thread (the shapes depend on
+// the cell size alone, and a cell at the mesh's own place would round lo + h): per shape and material
 // the element matrix in FP64 and with FP32 products ([(la DIM + q)(NPE DIM) + lb DIM + q2]), and the
 // macroscale response w B_la^T D ([(la DIM + q) NV + v]).  Shapes: tri3 2 x cell parity + element in
 // the cell, quad4 one, tet4 the tet's place in the hex.
@@ -450,10 +451,10 @@ __host__ __device__ constexpr int corner_bit(int cn, int d) {
 }
 
 template <int DIM, int NPE>
-__global__ void k_shape_consts(DevProblem P, double lo0, double lo1, double lo2, double h0, double h1, double h2, double* out) {
+__global__ void k_shape_consts(DevProblem P, double h0, double h1, double h2, double* out) {
   constexpr int ND = NPE * DIM, NV = (DIM == 2) ? 3 : 6;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double lo[3] = {lo0, lo1, lo2}, h[3] = {h0, h1, h2};
+  const double h[3] = {h0, h1, h2};
   for (int sh = 0; sh < shape_count(DIM, NPE); ++sh) {
     double x[NPE][DIM];
     for (int n = 0; n < NPE; ++n)
@@ -462,7 +463,7 @@ __global__ void k_shape_consts(DevProblem P, double lo0, double lo1, double lo2,
         if (DIM == 3) o = corner_bit(tet_corner(sh, n), d);
         else if (NPE == 4) o = (d == 0) ? (n == 1 || n == 2) : (n >= 2);
         else o = tri_corner(sh, n, d);
-        x[n][d] = __dadd_rn(lo[d], __dmul_rn((double)o, h[d]));
+        x[n][d] = o ? h[d] : 0.0;
       }
     for (int m = 0; m < 3; ++m) {
       double* ke = out + (size_t)(sh * 3 + m) * shape_doubles(DIM, NPE);
