@@ -132,7 +132,8 @@ int pg_debug_array(const pg_ctx* ctx, const char* name, int64_t* n, const void**
  *   "pcg_missing"       arrivals that the grid barriers of a solve's later launches wait for although
  *                       none will come (0: none): the solve runs into that limit, PG_ERR_DEVICE
  *   "fail_alloc"        which allocation of the context's working memory fails, counted from the
- *                       next one (0: none) */
+ *                       next one (0: none)
+ *   "fail_launch"       likewise which launch of pg_residual_norm */
 int pg_debug_set(pg_ctx* ctx, const char* name, int64_t value);
 void pg_destroy(pg_ctx* ctx);
 const char* pg_last_error(const pg_ctx* ctx);

@@ -773,8 +773,8 @@ int pg_debug_set(pg_ctx* c, const char* name, int64_t value) {
     (name[4] == 'w' ? c->pcg.wait_ms : c->pcg.missing) = (int)value;
     return 0;
   }
-  if (std::strcmp(name, "fail_alloc") == 0) {
-    c->fail_alloc = (int)value;
+  if (std::strcmp(name, "fail_alloc") == 0 || std::strcmp(name, "fail_launch") == 0) {
+    (name[5] == 'a' ? c->fail_alloc : c->fail_launch) = (int)value;
     return 0;
   }
   return set_err(c, PG_ERR_INPUT, "pg_debug_set: unknown name");
@@ -999,10 +999,23 @@ int pg_set_macro_strain(pg_ctx* c, const double* eps) {
 int pg_residual_norm(pg_ctx* c, double* out) {
   if (!c || !out) return PG_ERR_INPUT;
   if (!pg_resident(c)) return set_err(c, PG_ERR_STATE, "the context has no device residency (pg_upload it first)");
-  if (!c->h_norm && cudaMallocHost(&c->h_norm, sizeof(double)) != cudaSuccess)
+  if (!c->h_norm && cudaMallocHost(&c->h_norm, sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();   // (reported here; a later call's check is for its own launches)
+    c->h_norm = nullptr;
     return set_err(c, PG_ERR_DEVICE, "pinned norm allocation failed");
+  }
   const int nb = std::max(1, (int)(((long long)c->s.n_free + kNormBlock - 1) / kNormBlock));
-  k_norm<<<nb, kNormThreads, 0, c->stream>>>(c->P.Pf, c->s.n_free, c->d_red + 1, reinterpret_cast<unsigned*>(c->d_red), c->h_norm);
+  // (without its own status a launch that failed would leave the last call's value to be returned)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nb);
+  cfg.blockDim = dim3(kNormThreads);
+  cfg.stream = c->stream;
+  const bool fail = c->fail_launch > 0 && --c->fail_launch == 0;
+  if (fail || cudaLaunchKernelEx(&cfg, k_norm, (const double*)c->P.Pf, c->s.n_free, c->d_red + 1,
+                                 reinterpret_cast<unsigned*>(c->d_red), c->h_norm) != cudaSuccess) {
+    cudaGetLastError();
+    return set_err(c, PG_ERR_DEVICE, "residual norm: launch failed");
+  }
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, PG_ERR_DEVICE, "residual norm failed");
   *out = *c->h_norm;
   return 0;

@@ -54,6 +54,7 @@ struct pg_ctx {
   bool assembled = false;
   bool timed_last = false;   // the last assembly recorded every timing event (pg_kernel_times)
   int fail_alloc = 0;        // the allocation from here on that fails (pg_debug_set; 0: none)
+  int fail_launch = 0;       // likewise the residual norm's launch
   double prep_ms = -1.0;   // device time of the preprocessing passes (pg_create_prep_device), -1 if none ran
   // PG_KEEP_STATIC: the first CSR value of each block from which a later assembly can change
   // values (the rows of DOFs of nodes on cohesive elements; nnz when no value can change), and
