@@ -267,8 +267,7 @@ int pg_batch_wait(pg_batch* b, float* ms) {
   if (cudaEventSynchronize(b->t1) != cudaSuccess) return berr(b, PG_ERR_DEVICE, "batch assembly failed");
   if (ms) cudaEventElapsedTime(ms, b->t0, b->t1);
   const int herr = *b->h_err;
-  if (herr) return berr(b, (herr & pgd::ERR_NONFINITE) ? PG_ERR_NONFINITE : PG_ERR_DEVICE,
-                        "a context of the batch reported a device error (pg_last_error of each context has no detail)");
+  if (herr) return berr(b, PG_ERR_NONFINITE, "a context of the batch reported a device error (pg_last_error of each context has no detail)");
   return 0;
 }
 

@@ -386,7 +386,6 @@ int pg_upload(pg_ctx* c) {
   std::vector<int> re_off(s.ncut + 1, 0);
   for (int cc = 0; cc < s.ncut; ++cc) {
     const int nd = (s.cut_node_off[cc + 1] - s.cut_node_off[cc]) * dim;
-    c->max_nd = std::max(c->max_nd, nd);
     ke_off[cc + 1] = ke_off[cc] + (long long)nd * nd;
     re_off[cc + 1] = re_off[cc] + nd;
   }
@@ -449,8 +448,8 @@ int pg_upload(pg_ctx* c) {
 
   // ---- device residency
   pgd::DevProblem& P = c->P;
-  P.dim = dim; P.npe = s.npe; P.nvoigt = s.nvoigt;
-  P.n_nodes = n_nodes; P.ne = s.ne; P.ncut = s.ncut; P.n_dn = s.n_dn;
+  P.dim = dim; P.npe = s.npe;
+  P.ne = s.ne; P.ncut = s.ncut; P.n_dn = s.n_dn;
   P.n_free = s.n_free; P.n_const = s.n_const; P.subscale = s.desc.subscale;
   P.coh.law = s.coh.law; P.coh.nvar = s.coh.nvar; P.coh.sigma_c = s.coh.sigma_c; P.coh.delta_c1 = s.coh.delta_c1;
   P.coh.delta_c2 = s.coh.delta_c2; P.coh.delta_cn = s.coh.delta_cn; P.coh.delta_ct = s.coh.delta_ct; P.coh.q = s.coh.q;
@@ -506,10 +505,6 @@ int pg_upload(pg_ctx* c) {
       if (qp != s.cut_qp_off[cc + 1]) return set_err(c, PG_ERR_STATE, "internal: quadrature count mismatch");
       dq_off.push_back((int)dq_w.size());
     }
-    for (int cc = 0; cc < s.ncut; ++cc) {
-      c->max_cut_qp = std::max(c->max_cut_qp, dq_off[cc + 1] - dq_off[cc]);
-      c->max_cut_nodes = std::max(c->max_cut_nodes, s.cut_node_off[cc + 1] - s.cut_node_off[cc]);
-    }
     {
       // size classes: at most 8 points and 8 nodes (one fiber: tri3 + quad4 sub-elements), the rest
       std::vector<int> lists[2];
@@ -547,7 +542,6 @@ int pg_upload(pg_ctx* c) {
   PG_TRY(dalloc(c, (size_t)c->n_coh_qp, &c->d_zone));
   P.zone = c->d_zone;
   PG_TRY(upload(c, s.dn_node, &P.dn_node));
-  PG_TRY(upload(c, s.dn_nbr_off, &P.dn_nbr_off));
   PG_TRY(upload(c, nbr_mask, &P.dn_nbr_mask));
   PG_TRY(upload(c, s.dn_adj_off, &P.dn_adj_off));
   PG_TRY(upload(c, s.dn_adj, &P.dn_adj));
@@ -605,7 +599,6 @@ int pg_upload(pg_ctx* c) {
     PG_TRY(dalloc(c, (size_t)kc_off[n_ce], &dk));
     P.kcoh = dk;
     P.n_coh_el = n_ce;
-    P.n_coh_qp = c->n_coh_qp;
   }
   // row positions: free DOFs of the earlier neighbours of every neighbour slot
   {
@@ -932,8 +925,7 @@ int pg_assemble(pg_ctx* c, const double* U, double t_frac, int flags, double* Kf
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_err(c, PG_ERR_DEVICE, std::string("assembly failed: ") + cudaGetErrorString(e));
   c->assembled = true;
-  if (herr & pgd::ERR_NONFINITE) return set_err(c, PG_ERR_NONFINITE, "non-finite value in a cut-element matrix or vector");
-  if (herr) return set_err(c, PG_ERR_DEVICE, "scatter map inconsistency detected on the device");
+  if (herr) return set_err(c, PG_ERR_NONFINITE, "non-finite value in a cut-element matrix or vector");
   return 0;
 }
 

@@ -49,7 +49,6 @@ struct pg_ctx {
   double* d_red = nullptr;  // residual norm: the count of finished blocks, then their partials
   double* h_norm = nullptr; // its result (pinned host memory the kernel writes)
   long long cut_scratch = 0;   // doubles of the cut elements' set-up blocks (released after set-up)
-  int max_nd = 0;
   int n_coh_qp = 0;
   bool assembled = false;
   bool timed_last = false;   // the last assembly recorded every timing event (pg_kernel_times)
@@ -63,7 +62,6 @@ struct pg_ctx {
   double* kept[4] = {nullptr, nullptr, nullptr, nullptr};
   bool kept_fp32 = false, kept_valid = false;
   std::vector<int> fast_dn, slow_dn;
-  int max_cut_qp = 1, max_cut_nodes = 1;
   const int* cut_list[2] = {nullptr, nullptr};
   int n_cut_list[2] = {0, 0};
   int cut_cls_qp[2] = {1, 1}, cut_cls_nodes[2] = {1, 1};

@@ -22,7 +22,7 @@ constexpr int kMaxNodesCut = 32;  // element-local node slots (parent + enrichme
 enum { COH_NONE = 0, COH_BL = 1, COH_BLNU = 2, COH_XN = 3, COH_XNNU = 4, COH_OP = 5, COH_OPNU = 6, COH_OPAUG = 7, COH_OPNUAUG = 8,
        COH_TL = 9, COH_TLNU = 10, COH_STL = 11, COH_STLNU = 12 };
 enum { FLAG_FUNC = 1, FLAG_JAC = 2, FLAG_FP32 = 4 };
-enum { ERR_NONFINITE = 1, ERR_CUT_OVERFLOW = 2, ERR_BAD_SLOT = 4 };
+enum { ERR_NONFINITE = 1 };
 
 struct CohConst {
   int law, nvar;
@@ -32,8 +32,8 @@ struct CohConst {
 
 // Everything one assembly launch reads or writes, as device pointers.
 struct DevProblem {
-  int dim, npe, nvoigt;
-  int n_nodes, ne, ncut, n_dn;
+  int dim, npe;
+  int ne, ncut, n_dn;
   int n_free, n_const;
   int subscale;
   const double* Dd;   // D of the bulk materials (3 x 36): 0 matrix, 1 fiber, 2 bounding plies
@@ -68,7 +68,7 @@ struct DevProblem {
   const double* gmac;       // set-up only: macroscale-strain response of the cut elements
   // general rows (pg_rows.cuh): per node two int4 (gnd: gen_node's descriptor), its rows' static
   // image (stat, laid out like the CSR rows), the node id of each slot (stat_node) and the
-  // macroscale-strain response (stat_g, dim x nvoigt); the first n_gen_plain nodes are on no
+  // macroscale-strain response (stat_g, dim x Voigt components); the first n_gen_plain nodes are on no
   // cohesive element.  The bulk laws are linear elastic, so these do not depend on the state;
   // k_general_static forms them once at set-up.
   const int4* gnd;
@@ -80,7 +80,7 @@ struct DevProblem {
   double* isv_trial;
   uint8_t* zone;            // per cohesive qp: damage zone (0 compression, 1 loading, 2 softening, 3 failed)
   // row ownership
-  const int* dn_node; const int* dn_nbr_off; const uint8_t* dn_nbr_mask;  // free-DOF bits of each neighbour
+  const int* dn_node; const uint8_t* dn_nbr_mask;  // free-DOF bits of each neighbour
   const int* dn_adj_off; const int* dn_adj;      // adjacent (element << 5 | local node)
   const uint8_t* adj_slots;                      // cut elements' entries: neighbour slot of each element node
   int n_slow_dn;                                 // the general DOF nodes
@@ -96,8 +96,7 @@ struct DevProblem {
   //                 cut: offset into adj_slots), material (uncut)}
   //   aresd[entry]  uncut {element nodes (-1 padded)}; cut {cut element, its first node in cut_nodes, -, 0}
   const int4* gdesc; const int* growd; const int4* adesc; const int4* aresd;
-  // cohesive points
-  int n_coh_qp;
+  // cohesive elements
   int n_coh_el;                                  // cohesive elements
   const int* coh_gnode;                          // node id of every cohesive element's local node ('-' then '+', at coh_local_off)
   double* kcoh;                                  // per call: cohesive blocks B_ab and tractions t_a
@@ -346,24 +345,6 @@ __device__ __forceinline__ void load_node(const double* __restrict__ A, int node
   } else {
 #pragma unroll
     for (int d = 0; d < DIM; ++d) v[d] = __ldg(&A[(size_t)node * DIM + d]);
-  }
-}
-
-// Voigt B-matrix entry B(r, k*dim + q) for a node with gradient g (dim entries).
-template <typename T>
-__device__ inline T bmat(int dim, int r, int q, const T* g) {
-  if (dim == 2) {
-    if (r == 0) return q == 0 ? g[0] : T(0);
-    if (r == 1) return q == 1 ? g[1] : T(0);
-    return q == 0 ? g[1] : g[0];
-  }
-  switch (r) {
-    case 0: return q == 0 ? g[0] : T(0);
-    case 1: return q == 1 ? g[1] : T(0);
-    case 2: return q == 2 ? g[2] : T(0);
-    case 3: return q == 0 ? T(0) : (q == 1 ? g[2] : g[1]);
-    case 4: return q == 1 ? T(0) : (q == 0 ? g[2] : g[0]);
-    default: return q == 2 ? T(0) : (q == 0 ? g[1] : g[0]);
   }
 }
 

@@ -676,8 +676,6 @@ int pcg_reserve(pg_ctx* c, int nrhs) {
     std::vector<int> gci;
     if (dim == 3) pcg_groups<3>(s, w.stage_values, grp, gci, chunk);
     else pcg_groups<2>(s, w.stage_values, grp, gci, chunk);
-    for (const int4& d : grp)
-      if (grp_len(d.w) >= 0x1000000 - 1) return pg_set_err(c, PG_ERR_UNSUPPORTED, "a row of K_ff with 2^24 entries");
     const int ng = (int)grp.size(), nch = (int)chunk.size() - 1;
     // blocks: one per SM (the launch is cooperative), fewer when there are fewer chunks than
     // warps; contiguous chunk ranges of about equal nonzeros plus vector work
