@@ -214,7 +214,7 @@ int pg_residual_norm(pg_ctx* ctx, double* out);
 /* Jacobi-preconditioned conjugate gradients on K_ff of the last assembly (FP64, on the device).
  * d_b: nrhs right-hand sides of n_free entries each, one after another; d_x: initial guesses in,
  * solutions out (same layout).  Stops each right-hand side at ||b - K x|| <= rtol ||b|| (checked
- * every iteration on the device; the host looks every 16 iterations, so at most max_it + 15
+ * every iteration on the device; the host looks every 16 or 128 iterations (a launch), at most max_it + 15
  * iterations run).  Inner products are fixed-order reductions: a right-hand side's result does not
  * depend on the others solved with it.  iters / relres (host, nrhs entries, may be NULL) get each
  * right-hand side's iteration count and final relative residual.  PG_ERR_STATE if any right-hand

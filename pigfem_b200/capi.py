@@ -449,6 +449,8 @@ class Batch:
         return tuple(int(x) for x in best)
 
     def info(self) -> dict:
+        # (stencil_tile_threads: the threads of a block of rows; general_threads_per_block: always 1, the
+        # keys are kept for their readers; the chunks are work items of the three kinds)
         v = np.zeros(8, np.int64)
         self._check(load_library().pg_batch_info(self.h, _ptr(v)))
         keys = ("contexts", "elements", "stencil_tile_threads", "general_threads_per_block", "blocks_per_sm",

@@ -389,7 +389,7 @@ __device__ __forceinline__ bool block_product(const PcgArgs& a, PcgRing<M>& ring
 // One launch per round instead of five kernels per iteration: a 128 x 128 tri3 RVE with three
 // right-hand sides (39,614 rows) takes 11.4 us per iteration (five kernels: 36 us), of which the
 // three barriers with their scalars are about 5 us; 40^3 tet4 with six (219,807 rows, 9.7 M
-// nonzeros) 65 us (134 us), bound by the latency and L1 wavefronts of the gathers of p (48 bytes
+// nonzeros) 66 us (132 us), bound by the latency of the gathers of p (48 bytes
 // per lane) at 16 warps per SM.
 template <int NS, int M>
 __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_run(PcgArgs a, int first, int it0, int it1, unsigned arrived) {
